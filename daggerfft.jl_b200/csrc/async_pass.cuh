@@ -97,10 +97,10 @@ __global__ void __launch_bounds__(LB, MINB) axis_pass_async(const PassDesc d, co
     const StrideColC<V, CS> dense{buf + c};
     if constexpr (kPow2) {
       const YSwzCol<V, CS, R0> sw{buf + c};
-      static_stages<T, L, P, true, 3, 0, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>, StrideColC<V, CS>,
+      static_stages<T, L, P, 3, 0, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>, StrideColC<V, CS>,
                     StageTw<V>, Rs...>(d, t, dense, sw, dense, tw, 0, ob, cv);
     } else {
-      static_stages<T, L, P, true, 3, 0, DIR, 1, 1, 0, StrideColC<V, CS>, StrideColC<V, CS>, StrideColC<V, CS>,
+      static_stages<T, L, P, 3, 0, DIR, 1, 1, 0, StrideColC<V, CS>, StrideColC<V, CS>, StrideColC<V, CS>,
                     StageTw<V>, Rs...>(d, t, dense, dense, dense, tw, 0, ob, cv);
     }
     __syncthreads();  // the next iteration's copies refill the buffer of tile i-1

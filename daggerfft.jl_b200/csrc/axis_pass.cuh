@@ -23,11 +23,9 @@
 // The inverse transform runs the forward kernel on conjugated data
 // (IDFT(x) = conj(DFT(conj(x)))), with the 1/L scale folded into the store.
 //
-// Two kernels share the stage body:
-//   * axis_pass_static<T, FAST_IO, LB, L, P, R...>: radices known at compile
-//     time, every stage inlined and constant-folded (the hot path);
-//   * axis_pass_dynamic<T, EMAX>: radices read from the descriptor, one
-//     out-of-line function per radix (any 13-smooth length).
+// axis_pass_static<T, LB, L, P, R...> serves plain complex sides; the other
+// sides (real, r2r, Bluestein) and run-time radices run on the same stage
+// body in any_pass.cuh.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -95,14 +93,16 @@ struct PassDesc {
   int ld;                   // shared-memory elements reserved per column
   int inverse;              // 1: conjugate on load and on store
   int cfast;                // thread -> (column, butterfly) mapping
-  int epi;                  // 1: R2C half-length post-pass on the way out
+  int epi;                  // 1: R2C half-length post-pass on the way out; kEpiChirp: Bluestein
   long long Q;              // number of columns
   long long I;              // column split q -> (q % I, q / I)
   double scale;             // multiplier applied at the store
   const void* tw;           // L entries exp(-2 pi i m / L)
-  const void* tw2;          // epi: L+1 entries exp(-2 pi i m / (2L))
+  const void* tw2;          // epi 1: L+1 entries exp(-2 pi i m / (2L)); kEpiChirp: filter spectrum, L entries
   IoAny in, out;
 };
+
+constexpr int kEpiChirp = 2;  // PassDesc::epi of a one-launch Bluestein pass
 
 // Bank-conflict swizzle for the shared-memory exchange: one pad element per
 // 128 bytes of complex data.
@@ -187,169 +187,6 @@ __device__ __forceinline__ void r2r_store(T* p, long long b, long long sk, int N
   } else {  // K_DHT
     p[b + k * sk] = (v.x - v.y) * s;
   }
-}
-
-template <typename T>
-__device__ __forceinline__ typename cvec<T>::type load_raw(const IoAny& io, long long b, int k) {
-  typedef typename cvec<T>::type V;
-  const T z = (T)0;
-  switch (io.kind) {
-    case IO_CPLX:
-      return reinterpret_cast<const V*>(io.p)[b + k * io.sk];
-    case IO_REAL_PAIR: {
-      const T* p = reinterpret_cast<const T*>(io.p);
-      if (io.sk == 1) return *reinterpret_cast<const V*>(p + b + 2 * (long long)k);
-      return mk<V>(p[b + (2 * k) * io.sk], p[b + (2 * k + 1) * io.sk]);
-    }
-    case IO_REAL:
-      return mk<V>(reinterpret_cast<const T*>(io.p)[b + k * io.sk], z);
-    case IO_HERM_PAIR: {
-      // Z'_k = (A + B) + i conj(w^k) (A - B), A = X_k, B = conj(X_{n-k});
-      // the inverse FFT of Z' (length n) interleaves to 2n * x.
-      const V* p = reinterpret_cast<const V*>(io.p);
-      V A = p[b + k * io.sk];
-      V B = cconj(p[b + (io.n - k) * io.sk]);
-      if (k == 0) { A.y = (T)0; B.y = (T)0; }  // c2r ignores Im X_0 and Im X_{n}
-      V wk;
-      if (io.w) {
-        wk = cconj(ldg_c(reinterpret_cast<const V*>(io.w) + k));
-      } else {  // exp(+2 pi i k / (2n)), computed in the kernel
-        double sn, cs;
-        sincospi((double)k / (double)io.n, &sn, &cs);
-        wk = mk<V>((T)cs, (T)sn);
-      }
-      return cadd(cadd(A, B), cmul_pi(cmul(wk, csub(A, B))));
-    }
-    case IO_HERM_FULL: {
-      const V* p = reinterpret_cast<const V*>(io.p);
-      if (io.t_m > 0) {
-        // sub-axis of a four-step pair: element kf of the whole axis, whose
-        // column starts j rows before b, rows t_i apart
-        const long long j = (b % io.t_ia) / io.t_i;
-        const long long kf = j + (long long)io.t_m * k;
-        const long long b0 = b - j * io.t_i;
-        if (kf == 0) return mk<V>(p[b0].x, z);
-        if (2 * kf <= io.n) return p[b0 + kf * io.t_i];
-        return cconj(p[b0 + (io.n - kf) * io.t_i]);
-      }
-      if (k == 0) return mk<V>(p[b].x, z);  // c2r ignores Im X_0
-      if (2 * k <= io.n) return p[b + k * io.sk];
-      return cconj(p[b + (io.n - k) * io.sk]);
-    }
-    default: {  // IO_R2R
-      const T* p = reinterpret_cast<const T*>(io.p);
-      const V* w = reinterpret_cast<const V*>(io.w);
-      // a four-step sub-axis reads element kf of the whole axis (column
-      // base moved back by j rows, rows t_i apart)
-      long long bb = b, ss = io.sk;
-      int kk = k;
-      if (io.t_m > 0) {
-        const long long j = (b % io.t_ia) / io.t_i;
-        bb = b - j * io.t_i;
-        ss = io.t_i;
-        kk = (int)(j + (long long)io.t_m * k);
-      }
-      switch (io.r2r) {
-        case K_REDFT10: return r2r_load<T, K_REDFT10>(p, bb, ss, io.n, w, kk);
-        case K_RODFT10: return r2r_load<T, K_RODFT10>(p, bb, ss, io.n, w, kk);
-        case K_REDFT01: return r2r_load<T, K_REDFT01>(p, bb, ss, io.n, w, kk);
-        case K_RODFT01: return r2r_load<T, K_RODFT01>(p, bb, ss, io.n, w, kk);
-        case K_REDFT11: return r2r_load<T, K_REDFT11>(p, bb, ss, io.n, w, kk);
-        case K_RODFT11: return r2r_load<T, K_RODFT11>(p, bb, ss, io.n, w, kk);
-        case K_REDFT00: return r2r_load<T, K_REDFT00>(p, bb, ss, io.n, w, kk);
-        case K_RODFT00: return r2r_load<T, K_RODFT00>(p, bb, ss, io.n, w, kk);
-        default: return r2r_load<T, K_DHT>(p, bb, ss, io.n, w, kk);
-      }
-    }
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_raw(const IoAny& io, long long b, int k,
-                                          typename cvec<T>::type v, T s) {
-  typedef typename cvec<T>::type V;
-  switch (io.kind) {
-    case IO_CPLX:
-      reinterpret_cast<V*>(io.p)[b + k * io.sk] = cscale(v, s);
-      return;
-    case IO_TRUNC: {
-      // (a four-step sub-axis keeps the outputs whose whole-axis index fits)
-      const long long kf = io.t_m > 0 ? (b % io.t_ia) / io.t_i + (long long)io.t_m * k : (long long)k;
-      if (kf <= io.n) reinterpret_cast<V*>(io.p)[b + k * io.sk] = cscale(v, s);
-      return;
-    }
-    case IO_CPLX_TW: {
-      const long long j = (b % io.t_ia) / io.t_i;
-      const V w = ldg_c(reinterpret_cast<const V*>(io.w) +
-                        (long long)(((unsigned long long)j * (unsigned long long)k) % (unsigned long long)io.n));
-      reinterpret_cast<V*>(io.p)[b + k * io.sk] = cscale(cmul(v, w), s);
-      return;
-    }
-    case IO_REAL_PAIR: {
-      T* p = reinterpret_cast<T*>(io.p);
-      if (io.sk == 1) { *reinterpret_cast<V*>(p + b + 2 * (long long)k) = cscale(v, s); return; }
-      p[b + (2 * k) * io.sk] = v.x * s;
-      p[b + (2 * k + 1) * io.sk] = v.y * s;
-      return;
-    }
-    case IO_REAL:
-      reinterpret_cast<T*>(io.p)[b + k * io.sk] = v.x * s;
-      return;
-    default: {  // IO_R2R
-      T* p = reinterpret_cast<T*>(io.p);
-      const V* w = reinterpret_cast<const V*>(io.w);
-      long long bb = b, ss = io.sk;  // the whole axis, as for the load
-      int kk = k;
-      if (io.t_m > 0) {
-        const long long j = (b % io.t_ia) / io.t_i;
-        bb = b - j * io.t_i;
-        ss = io.t_i;
-        kk = (int)(j + (long long)io.t_m * k);
-      }
-      switch (io.r2r) {
-        case K_REDFT10: r2r_store<T, K_REDFT10>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_RODFT10: r2r_store<T, K_RODFT10>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_REDFT01: r2r_store<T, K_REDFT01>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_RODFT01: r2r_store<T, K_RODFT01>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_REDFT11: r2r_store<T, K_REDFT11>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_RODFT11: r2r_store<T, K_RODFT11>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_REDFT00: r2r_store<T, K_REDFT00>(p, bb, ss, io.n, w, kk, v, s); return;
-        case K_RODFT00: r2r_store<T, K_RODFT00>(p, bb, ss, io.n, w, kk, v, s); return;
-        default: r2r_store<T, K_DHT>(p, bb, ss, io.n, w, kk, v, s); return;
-      }
-    }
-  }
-}
-
-// Index along the whole axis of element k of the column at base b.
-__device__ __forceinline__ long long axis_index(const IoAny& io, long long b, int k) {
-  return io.t_m > 0 ? (b % io.t_ia) / io.t_i + (long long)io.t_m * k : (long long)k;
-}
-
-// Element access with the optional Bluestein chirp / filter multiply.
-template <typename T>
-__device__ __forceinline__ typename cvec<T>::type load_elem(const IoAny& io, long long b, int k) {
-  typedef typename cvec<T>::type V;
-  if (io.chirp) {
-    const long long n = axis_index(io, b, k);
-    if (n >= io.chirp_n) return mk<V>((T)0, (T)0);
-    return cmul(load_raw<T>(io, b, k), ldg_c(reinterpret_cast<const V*>(io.chirp) + n));
-  }
-  V v = load_raw<T>(io, b, k);
-  if (io.mul) v = cmul(v, ldg_c(reinterpret_cast<const V*>(io.mul) + axis_index(io, b, k)));
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ void store_elem(const IoAny& io, long long b, int k,
-                                           typename cvec<T>::type v, T s) {
-  typedef typename cvec<T>::type V;
-  if (io.chirp) {
-    const long long n = axis_index(io, b, k);
-    if (n >= io.chirp_n) return;
-    v = cmul(v, ldg_c(reinterpret_cast<const V*>(io.chirp) + n));
-  }
-  store_raw<T>(io, b, k, v, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -444,7 +281,7 @@ template <int BAR> __device__ __forceinline__ void stage_sync() {
 // CIN/COUT: the shared-memory views the stage reads and writes (they differ
 // when a stage moves a tile between a dense TMA buffer and a padded one).
 // toff: offset of this stage in a StageTw table (Ns - R_0).
-template <typename T, int R, int BMAX, bool FAST_IO, int SMEM_IO, int BAR, int DIR, class CIN, class COUT, class TW>
+template <typename T, int R, int BMAX, int SMEM_IO, int BAR, int DIR, class CIN, class COUT, class TW>
 __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int Ns, int ts, int toff,
                                            bool first, bool last, int t, const CIN& cin,
                                            const COUT& cout, const TW& tw, long long ib,
@@ -458,7 +295,7 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
   // table says so): only the r = 0 inputs are scaled here
   const bool fold = scaled_last_tw<TW>::value && DIR == 2 && last && !first;
   const T scale = DIR == 1 || fold ? (T)1 : (T)d.scale;
-  const bool to_global = SMEM_IO != 1 && last && !d.epi;
+  const bool to_global = SMEM_IO != 1 && last;
   const bool from_global = SMEM_IO == 0 && first;
   V v[BMAX][R];
 #pragma unroll
@@ -471,8 +308,7 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
         if (from_global) {
           V x;
           if (!cv) x = mk<V>((T)0, (T)0);
-          else if (FAST_IO) x = reinterpret_cast<const V*>(d.in.p)[ib + k * d.in.sk];
-          else x = load_elem<T>(d.in, ib, k);
+          else x = reinterpret_cast<const V*>(d.in.p)[ib + k * d.in.sk];
           if (inv) x.y = -x.y;
           v[b][r] = x;
         } else {
@@ -505,8 +341,7 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
             if (inv) y.y = -y.y;
             // SMEM_IO 2 (the fused slab pass) stores whole pencils: unit stride;
             // SMEM_IO 3 (the cp.async strided pass) rows d.out.sk apart
-            if (FAST_IO) reinterpret_cast<V*>(d.out.p)[ob + (SMEM_IO == 2 ? k : k * d.out.sk)] = cscale(y, scale);
-            else store_elem<T>(d.out, ob, k, y, scale);
+            reinterpret_cast<V*>(d.out.p)[ob + (SMEM_IO == 2 ? k : k * d.out.sk)] = cscale(y, scale);
           }
         } else if (SMEM_IO == 1 && last) {
           V y = v[b][r];
@@ -542,31 +377,13 @@ __device__ __forceinline__ ColCtx col_ctx(const PassDesc& d, int P) {
   return x;
 }
 
-// R2C post-pass over the half-length spectrum Z (length M) in shared memory:
-// X_k = E_k + w^k O_k, E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2.
-template <typename T>
-__device__ __forceinline__ void r2c_epilogue(const PassDesc& d, int P, const ColCtx& x,
-                                             const typename cvec<T>::type* col) {
-  typedef typename cvec<T>::type V;
-  const int M = d.L;
-  const V* w2 = reinterpret_cast<const V*>(d.tw2);
-  if (!x.cv) return;
-  for (int k = x.t; k <= M; k += P) {
-    V zk = col[swz<V>(k == M ? 0 : k)];
-    V zm = cconj(col[swz<V>(k == 0 ? 0 : M - k)]);
-    V e = cscale(cadd(zk, zm), (T)0.5);
-    V o = cscale(cmul_mi(csub(zk, zm)), (T)0.5);
-    store_elem<T>(d.out, x.ob, k, cadd(e, cmul(ldg_c(w2 + k), o)), (T)d.scale);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Static-plan kernel.
 // ---------------------------------------------------------------------------
 
 // Compile-time stage sequence.  The first stage reads CFIRST, the last
 // stage writes CLAST, every other access goes through CMID.
-template <typename T, int L, int P, bool FAST_IO, int SMEM_IO, int BAR, int DIR, int NS, int R0, int S, class CFIRST,
+template <typename T, int L, int P, int SMEM_IO, int BAR, int DIR, int NS, int R0, int S, class CFIRST,
           class CMID, class CLAST, class TW, int R, int... Rest>
 __device__ __forceinline__ void static_stages(const PassDesc& d, int t, const CFIRST& cf,
                                               const CMID& cm, const CLAST& cl, const TW& tw,
@@ -578,20 +395,20 @@ __device__ __forceinline__ void static_stages(const PassDesc& d, int t, const CF
   constexpr bool LAST = (sizeof...(Rest) == 0);
   constexpr int R0_ = FIRST ? R : R0;
   if constexpr (FIRST && LAST) {
-    stage_body<T, R, BM, FAST_IO, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, true, t, cf, cl, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, true, t, cf, cl, tw, ib, ob, cv);
   } else if constexpr (FIRST) {
-    stage_body<T, R, BM, FAST_IO, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, false, t, cf, cm, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, false, t, cf, cm, tw, ib, ob, cv);
   } else if constexpr (LAST) {
-    stage_body<T, R, BM, FAST_IO, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, true, t, cm, cl, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, true, t, cm, cl, tw, ib, ob, cv);
   } else {
-    stage_body<T, R, BM, FAST_IO, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, false, t, cm, cm, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, false, t, cm, cm, tw, ib, ob, cv);
   }
   if constexpr (sizeof...(Rest) > 0)
-    static_stages<T, L, P, FAST_IO, SMEM_IO, BAR, DIR, NS * R, R0_, S + 1, CFIRST, CMID, CLAST, TW, Rest...>(
+    static_stages<T, L, P, SMEM_IO, BAR, DIR, NS * R, R0_, S + 1, CFIRST, CMID, CLAST, TW, Rest...>(
         d, t, cf, cm, cl, tw, ib, ob, cv);
 }
 
-template <typename T, bool FAST_IO, int LB, int L, int P, int... Rs>
+template <typename T, int LB, int L, int P, int... Rs>
 __global__ void __launch_bounds__(LB) axis_pass_static(const PassDesc d) {
   typedef typename cvec<T>::type V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -599,57 +416,8 @@ __global__ void __launch_bounds__(LB) axis_pass_static(const PassDesc d) {
   const ColCtx x = col_ctx(d, P);
   const PadCol<V> col{sm + x.c * d.ld};
   const GlobalTw<V> tw{reinterpret_cast<const V*>(d.tw)};
-  static_stages<T, L, P, FAST_IO, 0, 0, 0, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(
+  static_stages<T, L, P, 0, 0, 0, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(
       d, x.t, col, col, col, tw, x.ib, x.ob, x.cv);
-  if (!FAST_IO && d.epi) r2c_epilogue<T>(d, P, x, col.p);
-}
-
-// ---------------------------------------------------------------------------
-// Dynamic-plan kernel (fallback for lengths without a static plan).
-// ---------------------------------------------------------------------------
-
-template <typename T, int R, int EMAX, bool CTW>
-__device__ __noinline__ void dyn_stage(const PassDesc& d, int s, int t, typename cvec<T>::type* col,
-                                       const typename cvec<T>::type* tw, long long ib, long long ob,
-                                       bool cv) {
-  typedef typename cvec<T>::type V;
-  const PadCol<V> c{col};
-  if constexpr (CTW) {
-    const ComputedTw<V> g{d.L};
-    stage_body<T, R, EMAX / R, false, 0, 0, 0>(d, d.L, d.P, d.ns[s], d.tws[s], 0, s == 0,
-                                             s == d.nst - 1, t, c, c, g, ib, ob, cv);
-  } else {
-    const GlobalTw<V> g{tw};
-    stage_body<T, R, EMAX / R, false, 0, 0, 0>(d, d.L, d.P, d.ns[s], d.tws[s], 0, s == 0,
-                                             s == d.nst - 1, t, c, c, g, ib, ob, cv);
-  }
-}
-
-// CTW: twiddles computed in the kernel instead of read from d.tw (no table).
-template <typename T, int EMAX, bool CTW = false>
-__global__ void __launch_bounds__(1024) axis_pass_dynamic(const PassDesc d) {
-  typedef typename cvec<T>::type V;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* sm = reinterpret_cast<V*>(smem_raw);
-  const ColCtx x = col_ctx(d, d.P);
-  V* col = sm + x.c * d.ld;
-  const V* tw = reinterpret_cast<const V*>(d.tw);
-  for (int s = 0; s < d.nst; ++s) {
-    switch (d.radix[s]) {
-      case 1: dyn_stage<T, 1, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 2: dyn_stage<T, 2, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 3: dyn_stage<T, 3, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 4: dyn_stage<T, 4, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 5: dyn_stage<T, 5, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 7: dyn_stage<T, 7, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 8: dyn_stage<T, 8, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 11: dyn_stage<T, 11, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 13: dyn_stage<T, 13, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      case 16: dyn_stage<T, 16, EMAX, CTW>(d, s, x.t, col, tw, x.ib, x.ob, x.cv); break;
-      default: break;
-    }
-  }
-  if (d.epi) r2c_epilogue<T>(d, d.P, x, col);
 }
 
 }  // namespace dfft

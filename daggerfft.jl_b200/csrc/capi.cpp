@@ -100,7 +100,8 @@ int dfft_plan_describe(dfft_plan plan, char* buf, size_t len) {
       char line[256];
       // the two passes of a four-step axis: twiddled store, then the split output
       const char* step = q.d.out.kind == dfft::IO_CPLX_TW || q.geom.tw_lo ? " four-step=1"
-                         : q.d.out.o1 > 0 || q.swap ? " four-step=2" : "";
+                         : q.d.out.o1 > 0 || q.swap ? " four-step=2"
+                         : q.d.epi == dfft::kEpiChirp ? " bluestein" : "";
       std::snprintf(line, sizeof line, "%s L=%d I=%lld O=%lld grid=%u block=%u smem=%zu radices=%s%s\n", kind,
                     q.d.L, q.d.I, q.d.I > 0 ? q.d.Q / q.d.I : 0LL, q.grid.x, q.block.x, q.smem,
                     rad.empty() ? "-" : rad.c_str(), step);

@@ -171,14 +171,15 @@ struct PassSpec {
   IoAny in{}, out{};         // pointers filled at execute time
   bool epi = false;          // R2C half-length post-pass
   bool fast_io = false;      // plain complex in/out
+  std::shared_ptr<DevTable> filter;  // Bluestein in one pass: FFT_L of the wrapped chirp over L
   int variant = VARIANT_AUTO;
   int C = 0;                 // columns per CTA (0: heuristic)
   std::vector<std::shared_ptr<DevTable>> keep;  // tables the IoAny sides point into
 };
 
-// Appends the passes of one axis: a single pass, or the two passes of
-// Bluestein's algorithm (via a scratch of Q*M complex elements) when no
-// single-pass kernel handles the length.  Returns the scratch bytes needed.
+// Appends the passes of one axis: a single pass (Bluestein's algorithm
+// included, when its convolution fits one CTA), or four-step passes through
+// a scratch.  Returns the scratch bytes needed.
 size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags, int src, int dst);
 
 // Builds a launchable pass; throws Error on unsupported sizes.

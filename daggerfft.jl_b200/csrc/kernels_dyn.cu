@@ -1,4 +1,5 @@
 // Dynamic-plan kernel instantiations (lengths without a static plan).
+#include "any_pass.cuh"
 #include "dfft_internal.h"
 
 namespace dfft {

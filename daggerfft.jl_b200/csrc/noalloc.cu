@@ -33,6 +33,7 @@
 //    stream and the array untouched.
 #include <mutex>
 #include "dfft.h"
+#include "any_pass.cuh"
 #include "dfft_internal.h"
 
 namespace dfft {

@@ -769,7 +769,7 @@ Pass make_pass(const PassSpec& s) {
   d.ld = ld;
   d.cfast = s.I > 1 ? 1 : 0;
   d.inverse = s.inverse;
-  d.epi = s.epi ? 1 : 0;
+  d.epi = s.filter ? kEpiChirp : s.epi ? 1 : 0;
   const long long Q = s.I * s.O;
   d.Q = Q;
   d.I = s.I;
@@ -863,6 +863,11 @@ Pass make_pass(const PassSpec& s) {
       // rows of at least 128 bytes for coalesced strided loads, ~256 threads
       C = s.dbl ? 8 : 16;
       while (C * P < 256 && C < 64) C *= 2;
+      // the kernels that stage the whole tile have their loads, stages and
+      // stores one after another: several CTAs per SM, not one of 1024
+      // threads, keep the memory busy (rows of 64 bytes still fill sectors)
+      if (!s.fast_io)
+        while (C * P > 512 && C * esz > 64) C /= 2;
     } else {
       C = 1;
       while (C * 2 * P <= 256) C *= 2;
@@ -879,7 +884,10 @@ Pass make_pass(const PassSpec& s) {
   auto tw = twiddle_table(s.dbl, L, 1, 0, L, false);
   p.tables.push_back(tw);
   d.tw = tw->p;
-  if (s.epi) {
+  if (s.filter) {
+    p.tables.push_back(s.filter);
+    d.tw2 = s.filter->p;
+  } else if (s.epi) {
     auto tw2 = twiddle_table(s.dbl, 2LL * L, 1, 0, L + 1, false);
     p.tables.push_back(tw2);
     d.tw2 = tw2->p;
@@ -1490,8 +1498,8 @@ static size_t add_direct_passes(std::vector<Pass>& out, const PassSpec& s, unsig
 //   X_k = w_k sum_n (x_n w_n) b_{k-n},  w_n = exp(s i pi n^2 / L),
 //   b_m = conj(w_m), s = -1 (forward) or +1 (inverse);
 // the convolution runs as FFT_M, a pointwise multiply by
-// Bhat = FFT_M(B) / M (B the wrapped b), and an inverse FFT_M, with M the
-// smallest 5-smooth length >= 2L-1.
+// Bhat = FFT_M(B) / M (B the wrapped b), and an inverse FFT_M, with M a
+// 5-smooth length >= 2L-1.
 // ---------------------------------------------------------------------------
 
 static int smooth5_at_least(int n) {
@@ -1519,6 +1527,25 @@ static std::shared_ptr<DevTable> upload(int dbl, const std::vector<long double>&
   return t;
 }
 
+// Convolution length for an N-point axis: of the 5-smooth lengths up to a
+// third above the smallest, the one with the least work (length x stages) in
+// a compiled kernel; the smallest one where none is compiled.
+static int bluestein_length(int dbl, int N) {
+  const int least = smooth5_at_least(2 * N - 1);
+  int best = least;
+  long long cost = -1;
+  for (long long m = least; m <= least + least / 3LL && m <= (1 << 14); ++m) {
+    const StaticPlan* sp = find_static(dbl, (int)m);
+    if (!sp || sp->P > sp->lb) continue;
+    const long long c = m * (sp->nst + 2);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = (int)m;
+    }
+  }
+  return best;
+}
+
 struct BluesteinTables {
   int M;
   std::shared_ptr<DevTable> chirp, bhat;
@@ -1538,7 +1565,7 @@ static BluesteinTables bluestein_tables(int dbl, int L, int sgn) {
     auto b = it->second.second.second.lock();
     if (a && b) return BluesteinTables{it->second.first, a, b};
   }
-  const int M = smooth5_at_least(2 * L - 1);
+  const int M = bluestein_length(dbl, L);
   const long double pi = acosl(-1.0L);
   // chirp w_n = exp(s i pi n^2 / L), n^2 reduced exactly modulo 2L
   std::vector<long double> wr(L), wi(L);
@@ -1631,6 +1658,35 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   BluesteinTables bt = bluestein_tables(s.dbl, L, s.inverse ? +1 : -1);
   const int M = bt.M;
   const size_t csz = s.dbl ? 16 : 8;
+  // both FFT_M, the filter and the two chirp multiplies on one tile in
+  // shared memory (kEpiChirp); 251 x 9800 ComplexF32 columns: two passes
+  // through a scratch of M-point columns took 102 us
+  {
+    PassSpec one = s;
+    one.L = M;
+    one.inverse = 0;
+    one.fast_io = false;
+    one.epi = false;
+    one.variant = VARIANT_AUTO;
+    one.C = 0;
+    one.in.chirp = one.out.chirp = bt.chirp->p;
+    one.in.chirp_n = one.out.chirp_n = L;
+    one.filter = bt.bhat;
+    one.keep.push_back(bt.chirp);
+    try {
+      Pass p = make_pass(one);
+      p.src = src;
+      p.dst = dst;
+      out.push_back(std::move(p));
+      return 0;
+    } catch (const Error& e) {
+      if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
+    }
+  }
+  // FFT_M does not fit one CTA: each FFT_M as a four-step pair, through two
+  // scratch halves: x * chirp -> S1 -> S2 (the spectrum), S2 * Bhat -> S1 ->
+  // out * chirp.  The last pass's sub-axis index k2 < M2 must stay below L
+  // (its column bases lie in the output).
   PassSpec a = s;
   a.L = M;
   a.inverse = 0;
@@ -1665,45 +1721,27 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   b.keep.push_back(bt.chirp);
   b.keep.push_back(bt.bhat);
   const size_t scratch = (size_t)(s.I * s.O) * (size_t)M * csz;
-  Pass pa, pb;
-  try {
-    pa = make_pass(a);
-    pb = make_pass(b);
-  } catch (const Error& e) {
-    if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
-    // FFT_M does not fit one CTA: each FFT_M as a four-step pair, through
-    // two scratch halves: x * chirp -> S1 -> S2 (the spectrum),
-    // S2 * Bhat -> S1 -> out * chirp.  The last pass's sub-axis index
-    // k2 < M2 must stay below L (its column bases lie in the output).
-    int M1 = 0, M2 = 0;
-    // the sub-axis index of a column must stay inside the column's extent
-    // on both sides (n1 < M1 rows of the input, k2 < M2 rows of the output)
-    long long ein = 0, eout = 0;
-    if (!four_step_extents(s, &ein, &eout) || !four_step_split(s.dbl, M, &M1, &M2) || M2 > eout || M1 > ein)
-      throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "length " + std::to_string(L) + " is too long for Bluestein here"};
-    Pass p[4];
-    four_step_pair(a, M1, M2, &p[0], &p[1]);
-    four_step_pair(b, M1, M2, &p[2], &p[3]);
-    p[0].src = src;
-    p[0].dst = BUF_CHIRP;
-    p[1].src = BUF_CHIRP;
-    p[1].dst = BUF_CHIRP;
-    p[1].dst_off = scratch;
-    p[2].src = BUF_CHIRP;
-    p[2].src_off = scratch;
-    p[2].dst = BUF_CHIRP;
-    p[3].src = BUF_CHIRP;
-    p[3].dst = dst;
-    for (Pass& q : p) out.push_back(std::move(q));
-    return 2 * scratch;
-  }
-  pa.src = src;
-  pa.dst = BUF_CHIRP;
-  pb.src = BUF_CHIRP;
-  pb.dst = dst;
-  out.push_back(std::move(pa));
-  out.push_back(std::move(pb));
-  return scratch;
+  int M1 = 0, M2 = 0;
+  // the sub-axis index of a column must stay inside the column's extent
+  // on both sides (n1 < M1 rows of the input, k2 < M2 rows of the output)
+  long long ein = 0, eout = 0;
+  if (!four_step_extents(s, &ein, &eout) || !four_step_split(s.dbl, M, &M1, &M2) || M2 > eout || M1 > ein)
+    throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "length " + std::to_string(L) + " is too long for Bluestein here"};
+  Pass p[4];
+  four_step_pair(a, M1, M2, &p[0], &p[1]);
+  four_step_pair(b, M1, M2, &p[2], &p[3]);
+  p[0].src = src;
+  p[0].dst = BUF_CHIRP;
+  p[1].src = BUF_CHIRP;
+  p[1].dst = BUF_CHIRP;
+  p[1].dst_off = scratch;
+  p[2].src = BUF_CHIRP;
+  p[2].src_off = scratch;
+  p[2].dst = BUF_CHIRP;
+  p[3].src = BUF_CHIRP;
+  p[3].dst = dst;
+  for (Pass& q : p) out.push_back(std::move(q));
+  return 2 * scratch;
 }
 
 }  // namespace dfft

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
       V* buf = bufs + b * bst;
       if constexpr (DIR == 1) {
         const StrideCol<V> padded{buf + (size_t)c * PS, 1};
-        static_stages<T, M, P, true, 1, NC, 1, 1, 1, 0, StrideCol<V>, PadCol<V>, PadCol<V>, StageTw<V>, Rs...>(
+        static_stages<T, M, P, 1, NC, 1, 1, 1, 0, StrideCol<V>, PadCol<V>, PadCol<V>, StageTw<V>, Rs...>(
             d, t, padded, pad, pad, tw, 0, 0, true);
         // post-pass: X_k of pencil cc, k = 0..M, into the consumed tile
         // buffer, dense: element e = cc*(M+1) + k
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
         }
         stage_sync<NC>();
         const StrideCol<V> padded{buf + (size_t)c * PS, 1};
-        static_stages<T, M, P, true, 1, NC, 2, 1, 1, 0, PadCol<V>, PadCol<V>, StrideCol<V>, StageTw<V>, Rs...>(
+        static_stages<T, M, P, 1, NC, 2, 1, 1, 0, PadCol<V>, PadCol<V>, StrideCol<V>, StageTw<V>, Rs...>(
             d, t, pad, pad, padded, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the producer's bulk store reads the tile next

@@ -387,17 +387,17 @@ __global__ void __launch_bounds__(LB, MINB)
         if constexpr (YX) {
           // out in pieces of rout elements, piece s of every pencil together
           const PieceCol<V> pc{buf, c, CS, __ffs(g.rout) - 1};
-          static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, PieceCol<V>,
+          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, PieceCol<V>,
                         TWT, Rs...>(dx, t, dense, sw, pc, tw, 0, 0, true);
         } else {
-          static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, StrideCol<V>,
+          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, StrideCol<V>,
                         TWT, Rs...>(dx, t, dense, sw, dense, tw, 0, 0, true);
         }
       } else {
         const int c = tid % CS, t = tid / CS;
         const StrideColC<V, CS> dense{buf + c};
         const YSwzCol<V, CS, R0> sw{buf + c};
-        static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>, StrideColC<V, CS>,
+        static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>, StrideColC<V, CS>,
                       TWT, Rs...>(dy, t, dense, sw, dense, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the buffer is next read (store) or written (load) by TMA
@@ -544,11 +544,11 @@ __global__ void __launch_bounds__(LB, MINB)
       if constexpr (kPow2) {
         // row-swizzled middle stages (bit-split addressing)
         const YSwzCol<V, CS, R0> sw{buf + c};
-        static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>,
+        static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>,
                       StrideColC<V, CS>, StageTw<V>, Rs...>(d, t, dense, sw, dense, tw, 0, 0, true);
       } else {
         // other lengths: the plain [row][column] tile (rows of 128 bytes)
-        static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, StrideColC<V, CS>,
+        static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, StrideColC<V, CS>,
                       StrideColC<V, CS>, StageTw<V>, Rs...>(d, t, dense, dense, dense, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the producer's TMA store reads the tile next

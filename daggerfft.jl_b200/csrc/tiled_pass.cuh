@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(LB, MINB)
       unsigned char* buf = bufs + b * bst;
       const In in{reinterpret_cast<const T*>(buf) + ib, d.in.n, w_in};
       const Out out{reinterpret_cast<T*>(buf) + ob, d.out.n, w_out};
-      static_stages<T, L, P, true, 1, NC, DIR, 1, 1, 0, In, PadCol<V>, Out, GlobalTw<V>, Rs...>(d, t, in, col, out,
+      static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, In, PadCol<V>, Out, GlobalTw<V>, Rs...>(d, t, in, col, out,
                                                                                             tw, 0, 0, true);
       fence_proxy_async_smem();  // the producer's store reads the tile next
       stage_sync<NC>();
