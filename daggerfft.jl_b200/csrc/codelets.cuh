@@ -7,9 +7,9 @@
 // (IDFT(x) = conj(DFT(conj(x)))), so only the forward sign is compiled.
 //
 // Radices: 2, 4 (butterflies), odd primes 3/5/7/11/13 (symmetric-pair form,
-// O(R^2/2) multiply-adds), composites 8 = 2x4, 16 = 4x4, 32 = 4x8,
-// 6 = 2x3, 10 = 2x5, 12 = 4x3, 15 = 3x5 (one Cooley-Tukey split in registers
-// with compile-time twiddles from roots.cuh).
+// O(R^2/2) multiply-adds), composites 8 = 2x4, 16 = 4x4, 24 = 4x6, 32 = 4x8,
+// 6 = 2x3, 10 = 2x5, 12 = 4x3, 14 = 2x7, 15 = 3x5 (one Cooley-Tukey split in
+// registers with compile-time twiddles from roots.cuh).
 #pragma once
 #include <cuda_runtime.h>
 #include "roots.cuh"
@@ -158,8 +158,20 @@ template <> struct Dft<7> : DftOdd<7> {};
 template <> struct Dft<11> : DftOdd<11> {};
 template <> struct Dft<13> : DftOdd<13> {};
 
-// R = R1*R2 in registers: n = R2*n1 + n2, k = k1 + R1*k2.
-template <int R1, int R2> struct DftComposite {
+// The first layer of a composite whose second half of inputs is zero
+// (zero-padded transforms): radix 2 and 4 over (a, 0) and (a, b, 0, 0).
+template <typename V> __device__ __forceinline__ void half_dft(V (&t)[2]) { t[1] = t[0]; }
+template <typename V> __device__ __forceinline__ void half_dft(V (&t)[4]) {
+  const V a = t[0], b = t[1], ib = cmul_mi(t[1]);
+  t[0] = cadd(a, b);
+  t[1] = cadd(a, ib);
+  t[2] = csub(a, b);
+  t[3] = csub(a, ib);
+}
+
+// R = R1*R2 in registers: n = R2*n1 + n2, k = k1 + R1*k2.  HALF: inputs
+// R/2 .. R-1 are zero (R1 is 2 or 4).
+template <int R1, int R2, bool HALF = false> struct DftComposite {
   template <typename V> __device__ __forceinline__ static void run(V (&x)[R1 * R2]) {
     constexpr int R = R1 * R2;
     V y[R2][R1];
@@ -168,7 +180,8 @@ template <int R1, int R2> struct DftComposite {
       V t[R1];
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1) t[n1] = x[R2 * n1 + n2];
-      Dft<R1>::run(t);
+      if constexpr (HALF) half_dft(t);
+      else Dft<R1>::run(t);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) y[n2][k1] = twiddle_const<R>(t[k1], n2 * k1);
     }
@@ -189,6 +202,16 @@ template <> struct Dft<32> : DftComposite<4, 8> {};
 template <> struct Dft<6> : DftComposite<2, 3> {};
 template <> struct Dft<10> : DftComposite<2, 5> {};
 template <> struct Dft<12> : DftComposite<4, 3> {};
+template <> struct Dft<14> : DftComposite<2, 7> {};
 template <> struct Dft<15> : DftComposite<3, 5> {};
+template <> struct Dft<24> : DftComposite<4, 6> {};
+
+// The same with a zero second half.
+template <int R> struct DftHalf;
+template <> struct DftHalf<8> : DftComposite<2, 4, true> {};
+template <> struct DftHalf<12> : DftComposite<4, 3, true> {};
+template <> struct DftHalf<16> : DftComposite<4, 4, true> {};
+template <> struct DftHalf<24> : DftComposite<4, 6, true> {};
+template <> struct DftHalf<32> : DftComposite<4, 8, true> {};
 
 }  // namespace dfft

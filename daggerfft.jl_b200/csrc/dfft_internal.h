@@ -124,6 +124,16 @@ struct TiledKernel {
   const void* fn;
 };
 const TiledKernel* find_tiled_kernel(int dbl, int L, int strided, int kind);
+// A compiled one-launch Bluestein pass (chirp_pass.cu): convolution length
+// M = r0 * r1, strided and contiguous kernels.
+struct ChirpKernel {
+  int dbl, M, r0, r1;
+  int P, cs;            // threads per column, columns per tile
+  const void *fn, *fn_contig;
+  size_t smem, smem_contig;
+};
+// The kernel with the shortest convolution for an N-point axis, or null.
+const ChirpKernel* find_chirp_kernel(int dbl, int N);
 
 // Fused forward or inverse 2-D C2C over dims 1 and 2 of an L x L x O array
 // (scales: 1 forward, 1/L per axis inverse) with launch variant v; throws

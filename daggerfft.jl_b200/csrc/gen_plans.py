@@ -1,8 +1,9 @@
 """Generates the static-plan kernel instantiations (plans_<dtype>_<k>.cu).
 
 For every 5-smooth length L (up to 4096 for single, 2048 for double
-precision) it picks a radix sequence with the fewest stages drawn from
-{2,3,4,5,6,8,10,12,15,16} (ties: most balanced), the thread count P per
+precision) and every 13-smooth one up to 1024 it picks a radix sequence with
+the fewest stages drawn from {2,3,4,5,6,8,10,12,15,16} (and 7, 11, 13, 14
+for the latter; ties: most balanced), the thread count P per
 column (one butterfly of the largest radix per thread and stage), and a
 __launch_bounds__ that leaves room for the per-thread registers.  Each entry
 is registered in a table the planner searches at plan time.
@@ -14,26 +15,41 @@ import math
 import os
 
 RADICES = [16, 15, 12, 10, 8, 6, 5, 4, 3, 2]
+# lengths with a factor 7, 11 or 13 (up to WIDE_LIMIT; longer ones take the
+# run-time-radix kernel, which is 4 times slower: the 25100 98-point pencils
+# of a ComplexF32 array take 58 us there and 14 us with radices 14 x 7)
+WIDE_RADICES = sorted(RADICES + [14, 13, 11, 7], reverse=True)
+WIDE_LIMIT = 1024
 NFILES = 6
 
 
-def smooth5(n):
-    for p in (2, 3, 5):
+def smooth(n, primes):
+    for p in primes:
         while n % p == 0:
             n //= p
     return n == 1
 
 
+def smooth5(n):
+    return smooth(n, (2, 3, 5))
+
+
+def compiled(n, lim):
+    """Lengths that get a static plan."""
+    return smooth5(n) if n > min(lim, WIDE_LIMIT) else smooth(n, (2, 3, 5, 7, 11, 13))
+
+
 def factorizations(n, maxr=16):
-    """All multisets of radices from RADICES whose product is n."""
+    """All multisets of radices whose product is n."""
     out = []
+    radices = RADICES if smooth5(n) else WIDE_RADICES
 
     def rec(rem, start, cur):
         if rem == 1:
             out.append(list(cur))
             return
-        for i in range(start, len(RADICES)):
-            r = RADICES[i]
+        for i in range(start, len(radices)):
+            r = radices[i]
             if r <= maxr and rem % r == 0:
                 cur.append(r)
                 rec(rem // r, i, cur)
@@ -80,7 +96,7 @@ def has_tma(dt, n):
     """C2C lengths that get the TMA-pipelined kernels (three tile buffers of
     at least 4 columns must fit in shared memory)."""
     esz = 8 if dt == "float" else 16
-    return 8 <= n and 3 * 4 * n * esz + 128 <= 227 * 1024 and n <= (1024 if dt == "float" else 512)
+    return smooth5(n) and 8 <= n and 3 * 4 * n * esz + 128 <= 227 * 1024 and n <= (1024 if dt == "float" else 512)
 
 
 def tma_bound(dt, lb):
@@ -106,7 +122,7 @@ def main():
     entries = []
     for dt, lim in (("float", 4096), ("double", 2048)):
         for n in range(1, lim + 1):
-            if not smooth5(n):
+            if not compiled(n, lim):
                 continue
             rad = choose(n)
             P = threads_per_column(n, rad)

@@ -6,7 +6,7 @@ double by the C++ compiler."""
 import mpmath as mp
 
 mp.mp.dps = 40
-RS = [3, 5, 6, 7, 8, 10, 11, 12, 13, 15, 16, 32]
+RS = [3, 5, 6, 7, 8, 10, 11, 12, 13, 14, 15, 16, 24, 32]
 
 print("// Generated by gen_roots.py -- do not edit.")
 print("#pragma once")

@@ -22,8 +22,12 @@ def _one_launch(transform, g, dims, **kw):
 
 
 @pytest.mark.parametrize("n,dtype", [
-    (17, np.complex64), (127, np.complex64), (251, np.complex64), (2039, np.complex64), (2053, np.complex64),
-    (8191, np.complex64), (19, np.complex128), (1021, np.complex128), (1031, np.complex128), (4093, np.complex128)])
+    # the longest prime of each two-radix convolution length, and the first past the last one
+    *[(n, np.complex64) for n in (17, 31, 47, 61, 89, 127, 191, 251, 383, 509, 521)],
+    *[(n, np.complex128) for n in (17, 31, 47, 61, 89, 127, 191, 251, 257)],
+    # compiled lengths of the general kernel, then its run-time radices
+    (2039, np.complex64), (2053, np.complex64), (8191, np.complex64),
+    (1021, np.complex128), (1031, np.complex128), (4093, np.complex128)])
 @pytest.mark.parametrize("strided", [False, True])
 def test_c2c_edges(n, dtype, strided):
     shape, dims = ((5, n, 3), (2,)) if strided else ((n, 7), (1,))
@@ -33,6 +37,17 @@ def test_c2c_edges(n, dtype, strided):
     F = dfft.fft(g, dims=dims)
     assert rel(to_np(F), oracle.fft(a, dims=dims)) <= tol_for(dtype)
     assert rel(to_np(dfft.ifft(F, dims=dims)), a) <= tol_for(dtype)
+
+
+@pytest.mark.parametrize("n", [14, 22, 26, 98, 182, 343, 1001, 1014])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_compiled_lengths_with_7_11_13(n, dtype):
+    a = rand((5, n, 7), dtype, seed=n)
+    g = to_gpu(a)
+    assert "dynamic" not in dfft.gpu_plan_transform(dfft.FFT(), g, (2,)).describe()
+    F = dfft.fft(g, dims=(2,))
+    assert rel(to_np(F), oracle.fft(a, dims=(2,))) <= tol_for(dtype)
+    assert rel(to_np(dfft.ifft(F, dims=(2,))), a) <= tol_for(dtype)
 
 
 @pytest.mark.parametrize("n", [31, 37, 158, 509])
