@@ -25,15 +25,17 @@
 
 namespace dfft {
 
-// Columns of the tile a thread helps to move, and its elements of them.
-// Strided axes (cfast): one column per thread, elements nthreads / C apart.
-// Contiguous axis: groups of G lanes walk whole columns.
+// Columns of the tile a thread helps to move, and its elements of them, so
+// that consecutive lanes touch consecutive memory of that side.  Columns
+// side by side (cfast): one column per thread, elements nthreads / C apart.
+// Unit stride along the column (the contiguous axis, and the output of a
+// four-step axis's first pass): groups of G lanes walk whole columns.
 struct TileLanes {
   int c, cstep, k, kstep;
 };
-__device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, int L) {
+__device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, const IoAny& io, int L) {
   const int tid = threadIdx.x, n = blockDim.x;
-  if (d.cfast) return TileLanes{tid % d.C, d.C, tid / d.C, n / d.C};
+  if (d.cfast && io.sk != 1) return TileLanes{tid % d.C, d.C, tid / d.C, n / d.C};
   int G = 1;
   while (G < 32 && G < L && G * 2 <= n) G *= 2;
   const int groups = n / G;  // a remainder of n mod G threads moves nothing
@@ -41,36 +43,37 @@ __device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, int L) {
   return TileLanes{g < groups ? g : d.C, groups, tid % G, G};
 }
 
-constexpr int kAnyBatch = 4;  // elements in flight per thread
+constexpr int kAnyBatch = 8;  // elements in flight per thread
+constexpr int kR2RBatch = 2;  // the r2r kinds: their maps are longer, and there are nine of them
 
 // Elements k, k + ks, ... < L of one column: get(k) from memory, times the
 // chirp or filter where the side has one (zero beyond the chirp), conjugated
 // for an inverse.
-template <typename T, class F>
+template <typename T, int N, class F>
 __device__ __forceinline__ void column_in(const IoAny& io, bool inv, long long j, typename cvec<T>::type* col, int k,
                                           int ks, int L, const F& get) {
   typedef typename cvec<T>::type V;
   const V* ch = reinterpret_cast<const V*>(io.chirp);
   const V* mu = reinterpret_cast<const V*>(io.mul);
   const long long tm = io.t_m > 0 ? io.t_m : 1;
-  for (; k < L; k += kAnyBatch * ks) {
-    V v[kAnyBatch];
+  for (; k < L; k += N * ks) {
+    V v[N];
 #pragma unroll
-    for (int u = 0; u < kAnyBatch; ++u) {
+    for (int u = 0; u < N; ++u) {
       const int e = k + u * ks;
       v[u] = mk<V>((T)0, (T)0);
       if (e < L && (!ch || j + tm * e < io.chirp_n)) v[u] = get(e);
     }
     if (ch || mu) {
 #pragma unroll
-      for (int u = 0; u < kAnyBatch; ++u) {
+      for (int u = 0; u < N; ++u) {
         const int e = k + u * ks;
         const long long n = j + tm * e;
         if (e < L && (!ch || n < io.chirp_n)) v[u] = cmul(v[u], ldg_c((ch ? ch : mu) + n));
       }
     }
 #pragma unroll
-    for (int u = 0; u < kAnyBatch; ++u) {
+    for (int u = 0; u < N; ++u) {
       const int e = k + u * ks;
       if (inv) v[u].y = -v[u].y;
       if (e < L) col[swz<V>(e)] = v[u];
@@ -78,24 +81,42 @@ __device__ __forceinline__ void column_in(const IoAny& io, bool inv, long long j
   }
 }
 
-// The way back: conjugation and chirp, then put(k, value).
-template <typename T, class F>
+// The way back: conjugation, chirp and factor(k), then put(k, value).  The
+// table reads of a batch go out together.
+struct NoFactor {};
+template <typename T, int N, class G, class F>
 __device__ __forceinline__ void column_out(const IoAny& io, bool inv, long long j, const typename cvec<T>::type* col,
-                                           int k, int ks, int n, F put) {
+                                           int k, int ks, int n, const G& factor, const F& put) {
   typedef typename cvec<T>::type V;
   const V* ch = reinterpret_cast<const V*>(io.chirp);
   const long long tm = io.t_m > 0 ? io.t_m : 1;
-  for (; k < n; k += kAnyBatch * ks) {
+  const long long last = io.chirp_n;
+  for (; k < n; k += N * ks) {
+    V v[N];
+    bool ok[N];
 #pragma unroll
-    for (int u = 0; u < kAnyBatch; ++u) {
+    for (int u = 0; u < N; ++u) {
       const int e = k + u * ks;
-      if (e >= n) continue;
-      if (ch && j + tm * e >= io.chirp_n) continue;
-      V v = col[swz<V>(e)];
-      if (inv) v.y = -v.y;
-      if (ch) v = cmul(v, ldg_c(ch + (j + tm * e)));
-      put(e, v);
+      ok[u] = e < n && (!ch || j + tm * e < last);
+      v[u] = mk<V>((T)0, (T)0);
+      if (ok[u]) v[u] = col[swz<V>(e)];
+      if (inv) v[u].y = -v[u].y;
     }
+    if (ch) {
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        if (ok[u]) v[u] = cmul(v[u], ldg_c(ch + (j + tm * (k + u * ks))));
+    }
+    if constexpr (!std::is_same<G, NoFactor>::value) {
+      V f[N];
+#pragma unroll
+      for (int u = 0; u < N; ++u) f[u] = factor(ok[u] ? k + u * ks : k);
+#pragma unroll
+      for (int u = 0; u < N; ++u) v[u] = cmul(v[u], f[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if (ok[u]) put(k + u * ks, v[u]);
   }
 }
 
@@ -130,7 +151,7 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
   typedef typename cvec<T>::type V;
   __builtin_assume(__isShared(sm));
   const IoAny& io = d.in;
-  const TileLanes ln = tile_lanes(d, L);
+  const TileLanes ln = tile_lanes(d, io, L);
   const bool inv = d.inverse != 0;
   const V* pc = reinterpret_cast<const V*>(io.p);
   const T* pr = reinterpret_cast<const T*>(io.p);
@@ -145,7 +166,7 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
     // index along the whole axis of the column's element 0 (four-step sub-axes)
     const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
     V* col = sm + (size_t)c * d.ld;
-    auto in = [&](auto get) { column_in<T>(io, inv, j, col, ln.k, ln.kstep, L, get); };
+    auto in = [&](auto get) { column_in<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, get); };
     switch (io.kind) {
       case IO_CPLX:
         in([=](int k) { return pc[b + k * sk]; });
@@ -180,6 +201,7 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
       }
       default: {
         const WholeAxis a = whole_axis(io, b);
+        auto in = [&](auto get) { column_in<T, kR2RBatch>(io, inv, j, col, ln.k, ln.kstep, L, get); };
 #define DFFT_R2R_IN(KIND) \
   case KIND: in([=](int k) { return r2r_load<T, KIND>(pr, a.b, a.s, io_n, w, a.at(k)); }); break;
         switch (io.r2r) {
@@ -198,7 +220,7 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
   typedef typename cvec<T>::type V;
   __builtin_assume(__isShared(sm));
   const IoAny& io = d.out;
-  const TileLanes ln = tile_lanes(d, L);
+  const TileLanes ln = tile_lanes(d, io, L);
   const bool inv = d.inverse != 0 || d.epi == kEpiChirp;
   V* pc = reinterpret_cast<V*>(io.p);
   T* pr = reinterpret_cast<T*>(io.p);
@@ -211,7 +233,7 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
     const long long b = column_base(io, d.I, q);
     const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
     const V* col = sm + (size_t)c * d.ld;
-    auto out = [&](int n, auto put) { column_out<T>(io, inv, j, col, ln.k, ln.kstep, n, put); };
+    auto out = [&](int n, auto put) { column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, n, NoFactor{}, put); };
     if (d.epi == 1) {
       // R2C post-pass over the half-length spectrum Z (length M = L):
       // X_k = E_k + w^k O_k, E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2
@@ -238,15 +260,12 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
         break;
       }
       case IO_CPLX_TW: {
-        // times w[(jj * k) mod n], stepped along the thread's elements
-        const unsigned n = (unsigned)io.n;
-        const unsigned long long jj = (unsigned long long)((b % io.t_ia) / io.t_i);
-        const unsigned step = (unsigned)((jj * (unsigned)ln.kstep) % n);
-        unsigned m = (unsigned)((jj * (unsigned)ln.k) % n);
-        out(L, [=](int k, V v) mutable {
-          pc[b + k * sk] = cscale(cmul(v, ldg_c(w + m)), s);
-          m = m >= n - step ? m - (n - step) : m + step;
-        });
+        const unsigned jj = (unsigned)((b % io.t_ia) / io.t_i);
+        const auto twiddle = [=](int k) {
+          const unsigned m = jj * (unsigned)k;
+          return cmul(ldg_c(w + m % kTwSplit), ldg_c(w + kTwSplit + m / kTwSplit));
+        };
+        column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, twiddle, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
         break;
       }
       case IO_REAL_PAIR:
@@ -262,6 +281,9 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
       default: {
         const WholeAxis a = whole_axis(io, b);
         const int N = io.n;
+        auto out = [&](int n, auto put) {
+          column_out<T, kR2RBatch>(io, inv, j, col, ln.k, ln.kstep, n, NoFactor{}, put);
+        };
 #define DFFT_R2R_OUT(KIND) \
   case KIND: out(L, [=](int k, V v) { r2r_store<T, KIND>(pr, a.b, a.s, N, w, a.at(k), v, s); }); break;
         switch (io.r2r) {
@@ -290,9 +312,13 @@ __device__ __forceinline__ void tile_filter(const PassDesc& d, typename cvec<T>:
 
 // Static radices.  The stages run forward on the tile (conjugation and scale
 // belong to the two ends); thread -> (column, butterfly lane) as in
-// axis_pass_static.
-template <typename T, int LB, int L, int P, int... Rs>
-__global__ void __launch_bounds__(LB) axis_pass_any(const __grid_constant__ PassDesc d) {
+// axis_pass_static.  CHIRP: Bluestein.  (The second copy of the stages is
+// spelled out: a loop over the two FFTs around one copy, entered once by the
+// other sides, spilled 300 to 900 bytes a thread: 35 us for 1024 columns of
+// 1024 ComplexF32 points.  One CTA per SM in the launch bounds: without it
+// the double-precision kernels are held to 64 registers.)
+template <typename T, int LB, bool CHIRP, int L, int P, int... Rs>
+__global__ void __launch_bounds__(LB, 1) axis_pass_any(const __grid_constant__ PassDesc d) {
   typedef typename cvec<T>::type V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* sm = reinterpret_cast<V*>(smem_raw);
@@ -303,12 +329,13 @@ __global__ void __launch_bounds__(LB) axis_pass_any(const __grid_constant__ Pass
   const GlobalTw<V> tw{reinterpret_cast<const V*>(d.tw)};
   tile_load<T>(d, sm, L);
   __syncthreads();
-  for (int half = 0;; ++half) {
-    static_stages<T, L, P, 1, 0, 1, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(
-        d, t, col, col, col, tw, 0, 0, true);
-    if (half || d.epi != kEpiChirp) break;
+  static_stages<T, L, P, 1, 0, 1, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(d, t, col, col, col,
+                                                                                             tw, 0, 0, true);
+  if constexpr (CHIRP) {
     tile_filter<T>(d, col.p, t, P, L);
     __syncthreads();
+    static_stages<T, L, P, 1, 0, 1, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(d, t, col, col, col,
+                                                                                               tw, 0, 0, true);
   }
   tile_store<T>(d, sm, L);
 }

@@ -45,9 +45,11 @@ enum IoKind : int {
   IO_HERM_FULL = 4,  // load only: odd-length C2R, Hermitian mirror
   IO_TRUNC = 5,      // store only: complex, keep k <= n
   IO_R2R = 6,        // FFTW r2r kind `r2r` on real data of extent n
-  IO_CPLX_TW = 7     // store only: complex times w[(j * k) mod n], j = (b mod t_ia) / t_i
-                     // (the twiddle between the two passes of a four-step axis)
+  IO_CPLX_TW = 7     // store only: complex times W_n^(j k), j = (b mod t_ia) / t_i (the twiddle
+                     // between the two passes of a four-step axis, j k < n); w holds W_n^m
+                     // for m < kTwSplit, then W_n^(kTwSplit m) for kTwSplit m < n
 };
+constexpr int kTwSplit = 1024;
 
 // FFTW r2r kind numbers (fftw_r2r_kind).
 enum : int { K_DHT = 2, K_REDFT00 = 3, K_REDFT01 = 4, K_REDFT10 = 5, K_REDFT11 = 6,
@@ -66,13 +68,13 @@ struct IoAny {
   const void* chirp;
   const void* mul;
   int chirp_n;
-  // Two-level column split of the outer index (four-step output): with
+  // Two-level column split of the outer index (four-step input): with
   // o1 > 0 the column base is (qo mod o1) * so + (qo / o1) * so2.
   long long o1, so2;
   // Sub-axis of a four-step pair: the column at base b holds elements
-  // j + t_m * k of the whole axis, j = (b mod t_ia) / t_i.  IO_CPLX_TW
-  // multiplies by w[(j * k) mod n]; with t_m > 0 the chirp and mul tables
-  // are indexed by j + t_m * k (Bluestein around a four-step pair).
+  // j + t_m * k of the whole axis, j = (b mod t_ia) / t_i.  With t_m > 0 the
+  // chirp and mul tables are indexed by j + t_m * k (Bluestein around a
+  // four-step pair).
   long long t_i, t_ia;
   int t_m;
 };

@@ -1,6 +1,9 @@
-// Instantiations of the one-launch Bluestein pass for plain complex axes
-// (axis_pass_chirp) and their launch shapes, shortest convolution first.
+// Instantiations of the one-launch Bluestein passes, shortest convolution
+// first: plain complex axes (axis_pass_chirp) with their launch shapes, and
+// the general one-tile kernel (axis_pass_any) for the other sides and the
+// longer convolutions.
 #define DFFT_PACKED_F32 1  // issue-bound butterflies
+#include "any_pass.cuh"
 #include "chirp_pass.cuh"
 #include "dfft_internal.h"
 
@@ -51,6 +54,35 @@ static const ChirpKernel kChirpKernels[] = {
 const ChirpKernel* find_chirp_kernel(int dbl, int N) {
   for (const ChirpKernel& k : kChirpKernels)
     if (k.dbl == dbl && k.M >= 2 * N - 1) return &k;
+  return nullptr;
+}
+
+// The general kernel: dtype, launch bound, length, threads per column, radices
+#define DFFT_CHIRP_ANY(X)                                                                              \
+  X(float, 0, 1024, 64, 8, 8, 8) X(float, 0, 1024, 96, 8, 12, 8) X(float, 0, 1024, 128, 8, 16, 8)      \
+  X(float, 0, 512, 192, 12, 12, 16) X(float, 0, 1024, 256, 16, 16, 16) X(float, 0, 1024, 384, 48, 6, 8, 8) \
+  X(float, 0, 1024, 512, 64, 8, 8, 8) X(float, 0, 1024, 768, 64, 12, 8, 8)                             \
+  X(float, 0, 1024, 1024, 64, 16, 8, 8) X(float, 0, 1024, 1536, 128, 12, 16, 8)                        \
+  X(float, 0, 1024, 2048, 128, 16, 16, 8) X(float, 0, 1024, 3072, 256, 12, 16, 16)                     \
+  X(float, 0, 1024, 4096, 256, 16, 16, 16)                                                             \
+  X(double, 1, 512, 64, 8, 8, 8) X(double, 1, 512, 96, 8, 12, 8) X(double, 1, 512, 128, 8, 16, 8)      \
+  X(double, 1, 512, 192, 12, 12, 16) X(double, 1, 512, 256, 16, 16, 16) X(double, 1, 512, 384, 48, 6, 8, 8) \
+  X(double, 1, 512, 512, 64, 8, 8, 8) X(double, 1, 512, 768, 64, 12, 8, 8)                             \
+  X(double, 1, 512, 1024, 64, 16, 8, 8) X(double, 1, 512, 1536, 128, 12, 16, 8)                        \
+  X(double, 1, 512, 2048, 128, 16, 16, 8)
+
+#define INST(T, DBL, LB, L, P, ...) \
+  template __global__ void axis_pass_any<T, LB, true, L, P, __VA_ARGS__>(const __grid_constant__ PassDesc);
+DFFT_CHIRP_ANY(INST)
+#undef INST
+
+#define ENTRY(T, DBL, LB, L, P, ...) {DBL, L, P, LB, {__VA_ARGS__}, (const void*)&axis_pass_any<T, LB, true, L, P, __VA_ARGS__>},
+static const ChirpAnyKernel kChirpAny[] = {DFFT_CHIRP_ANY(ENTRY)};
+#undef ENTRY
+
+const ChirpAnyKernel* find_chirp_any(int dbl, int least) {
+  for (const ChirpAnyKernel& k : kChirpAny)
+    if (k.dbl == dbl && k.L >= least) return &k;
   return nullptr;
 }
 

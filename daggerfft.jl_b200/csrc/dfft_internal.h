@@ -6,6 +6,7 @@
 #include <string>
 #include <vector>
 #include "async_pass.cuh"
+#include "fourstep_pass.cuh"
 #include "mixed_pass.cuh"
 
 namespace dfft {
@@ -38,13 +39,6 @@ std::shared_ptr<DevTable> twiddle_table(int dbl, long long D, long long a, long 
 // One kernel launch of a plan.
 enum BufId : int { BUF_IN = 0, BUF_OUT = 1, BUF_WORK = 2, BUF_CHIRP = 3 };
 
-// Axis swap of the last four-step pass (transpose_pass.cu): element
-// (i, a, b, o) of an I x A x B x O array moves to (i, b, a, o).
-struct SwapGeom {
-  long long I, A, B, O;
-};
-const void* swap_axes_kernel(int dbl, bool tiled);
-
 struct Pass {
   PassDesc d{};
   const void* fn = nullptr;
@@ -53,6 +47,9 @@ struct Pass {
   int src = BUF_IN, dst = BUF_OUT;
   size_t src_off = 0, dst_off = 0;  // byte offsets into those buffers
   bool is_static = false;
+  int four_step = 0;  // 1, 2: first / second pass of a four-step axis
+  bool fsfirst = false;  // four_step_first
+  FourStepGeom fsgeom{};
   // persistent pipelined pass (bulk copies); tma: strided, tensor
   // {I*xscale, L, O} of 8-byte elements
   bool pipe = false;
@@ -82,8 +79,6 @@ struct Pass {
   // MODE 2): the y-phase reads `in` through a map {tI2, tL2, tO2} and writes
   // the plain intermediate {L, L, nslab} (in `in` when cols_mid_in, else
   // in `out`), which the x-phase then reads
-  bool swap = false;     // swap_axes_* (the last pass of a fast four-step axis)
-  SwapGeom swg{};
   bool cols = false;
   bool cols_mid_in = false;
   long long tI2 = 0, tL2 = 0, tO2 = 0;
@@ -134,6 +129,21 @@ struct ChirpKernel {
 };
 // The kernel with the shortest convolution for an N-point axis, or null.
 const ChirpKernel* find_chirp_kernel(int dbl, int N);
+// A compiled four_step_first (fourstep_pass.cu) of length M = r0 * r1, or null.
+struct FourStepKernel {
+  int dbl, M, r0, r1;
+  int P, cs;  // threads and columns per tile
+  const void* fn;
+  size_t smem;
+};
+const FourStepKernel* find_four_step_kernel(int dbl, int M);
+// The general one-tile kernel's Bluestein form (chirp_pass.cu), shortest
+// compiled convolution of at least `least` points, or null.
+struct ChirpAnyKernel {
+  int dbl, L, P, lb, radix[4];
+  const void* fn;
+};
+const ChirpAnyKernel* find_chirp_any(int dbl, int least);
 
 // Fused forward or inverse 2-D C2C over dims 1 and 2 of an L x L x O array
 // (scales: 1 forward, 1/L per axis inverse) with launch variant v; throws

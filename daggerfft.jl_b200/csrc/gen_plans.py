@@ -140,7 +140,7 @@ def main():
             for (_, n, P, rad, lb) in ch:
                 rs = ",".join(str(r) for r in rad)
                 lines.append(f"template __global__ void axis_pass_static<{dt},{lb},{n},{P},{rs}>(const PassDesc);")
-                lines.append(f"template __global__ void axis_pass_any<{dt},{lb},{n},{P},{rs}>(const __grid_constant__ PassDesc);")
+                lines.append(f"template __global__ void axis_pass_any<{dt},{lb},false,{n},{P},{rs}>(const __grid_constant__ PassDesc);")
                 if has_tma(dt, n):
                     tlb = tma_bound(dt, lb)
                     for cg, cs in (("false", strided_c(dt, n, P, tlb)), ("true", 0)):
@@ -162,7 +162,7 @@ def main():
                 lines.append(
                     f"  {{{n}, {P}, {len(rad)}, {radarr}, {lb}, "
                     f"(const void*)&axis_pass_static<{dt},{lb},{n},{P},{rs}>, "
-                    f"(const void*)&axis_pass_any<{dt},{lb},{n},{P},{rs}>, {ps}, {pc}, {tlb}, "
+                    f"(const void*)&axis_pass_any<{dt},{lb},false,{n},{P},{rs}>, {ps}, {pc}, {tlb}, "
                     f"{cs if has_tma(dt, n) else 0}}},")
             lines.append("};")
             lines.append(f"const int kPlansCount_{tag}_{fi} = {len(ch)};")

@@ -675,6 +675,19 @@ Pass make_pass(const PassSpec& s) {
   const size_t smax = max_smem_per_block();
   const StaticPlan* sp = find_static(s.dbl, L);
   if (sp && sp->P > sp->lb) sp = nullptr;
+  StaticPlan chirp{};  // a Bluestein pass: its own set of compiled lengths
+  if (s.filter) {
+    sp = nullptr;
+    const ChirpAnyKernel* k = find_chirp_any(s.dbl, L);
+    if (k && k->L == L) {
+      chirp.L = L;
+      chirp.P = k->P;
+      while (chirp.nst < 4 && k->radix[chirp.nst]) chirp.radix[chirp.nst] = k->radix[chirp.nst], ++chirp.nst;
+      chirp.lb = k->lb;
+      chirp.any = k->fn;
+      sp = &chirp;
+    }
+  }
   int variant = s.variant;
   if (variant == VARIANT_AUTO) {
     // strided axes: the producer-fed kernel for passes of 16 MiB and more
@@ -767,7 +780,8 @@ Pass make_pass(const PassSpec& s) {
   int ld = swz_host(L - 1, esz) + 1;
   if ((ld & 1) == 0) ld += 1;
   d.ld = ld;
-  d.cfast = s.I > 1 ? 1 : 0;
+  // (with a two-level input of unit stride, columns lie side by side too)
+  d.cfast = s.I > 1 || (s.in.o1 > 0 && s.in.so == 1) ? 1 : 0;
   d.inverse = s.inverse;
   d.epi = s.filter ? kEpiChirp : s.epi ? 1 : 0;
   const long long Q = s.I * s.O;
@@ -866,8 +880,10 @@ Pass make_pass(const PassSpec& s) {
       // the kernels that stage the whole tile have their loads, stages and
       // stores one after another: several CTAs per SM, not one of 1024
       // threads, keep the memory busy (rows of 64 bytes still fill sectors)
+      // and short passes get two CTAs per SM while rows fill a sector (2^20
+      // ComplexF32: 128 CTAs of 8 columns against 256 of 4)
       if (!s.fast_io)
-        while (C * P > 512 && C * esz > 64) C /= 2;
+        while ((C * P > 512 && C * esz > 64) || (C * esz > 32 && (Q + C - 1) / C < 2 * sm_count())) C /= 2;
     } else {
       C = 1;
       while (C * 2 * P <= 256) C *= 2;
@@ -881,6 +897,17 @@ Pass make_pass(const PassSpec& s) {
     if (c2 < C) C = c2;
   }
   d.C = C;
+  if (d.cfast) {
+    // columns side by side: with fewer than a bank row of them, spread them
+    // evenly over it, so that a warp's C columns x 32/C rows do not collide
+    const int row = 128 / esz;
+    if (C > 1 && C < row && (C & (C - 1)) == 0) {
+      const size_t room = smax / ((size_t)C * esz);
+      int l = swz_host(L - 1, esz) + 1;
+      while (l % row != row / C) ++l;
+      if ((size_t)l <= room) d.ld = l;
+    }
+  }
   auto tw = twiddle_table(s.dbl, L, 1, 0, L, false);
   p.tables.push_back(tw);
   d.tw = tw->p;
@@ -896,7 +923,7 @@ Pass make_pass(const PassSpec& s) {
   if (nblk > 0x7fffffffLL) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "too many columns for one launch"};
   p.grid = dim3((unsigned)nblk);
   p.block = dim3((unsigned)(C * P));
-  p.smem = (size_t)C * col_bytes;
+  p.smem = (size_t)C * d.ld * esz;
   return p;
 }
 
@@ -1142,12 +1169,12 @@ cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream,
     void* args[] = {&d, &tin, &tout, &g};
     return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
   }
-  if (p.swap) {
-    const void* a = in;
-    void* b = out;
-    SwapGeom g = p.swg;
-    void* args[] = {&a, &b, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, 0, stream);
+  if (p.fsfirst) {
+    const void* ip = in;
+    void* op = out;
+    FourStepGeom g = p.fsgeom;
+    void* args[] = {&ip, &op, &g};
+    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
   }
   if (p.slab) {
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15)
@@ -1203,10 +1230,14 @@ namespace dfft {
 // Four-step decomposition of a complex axis that no single pass handles:
 // L = L1 * L2, n = n1 + L1 n2, k = k2 + L2 k1,
 //   X[k2 + L2 k1] = sum_n1 W_L1^(n1 k1) [ W_L^(n1 k2) sum_n2 x[n1 + L1 n2] W_L2^(n2 k2) ].
-// Pass A: L2-point transforms along the sub-axis of stride I*L1 (columns
-// (i, n1, o)), into a scratch in the same layout, times W_L^(n1 k2) on the
-// way out; pass B: L1-point transforms along stride I (columns (i, k2, o)),
-// written to position k2 + L2 k1 (the output's two-level column split).
+// Pass A: L2-point transforms along the sub-axis n2 (columns (i, n1, o), side
+// by side), times W_L^(n1 k2) on the way out, into a scratch with the two
+// sub-axes swapped: (i, k2, n1, o).  Pass B: L1-point transforms along n1 of
+// the columns (i, k2, o), whose outputs (i, k2, k1, o) are the axis in
+// order: for plain complex outputs an ordinary strided pass on its pipelined
+// kernel.  (Without the swap in pass A, B reads pencils and writes elements
+// L2 apart, or a third pass swaps: 2^20 ComplexF32 56 and 48 us, against
+// 23 us for this form.)
 // Each factor runs as one pass: a static plan, or the dynamic kernel for
 // lengths up to 4096 with prime factors up to 13 that fit one CTA.  Splits
 // with two static factors come first, then the most balanced one.
@@ -1227,7 +1258,25 @@ static int four_step_factor(int dbl, int n) {
   return P <= 1024 ? VARIANT_DYNAMIC : 0;
 }
 
-static bool four_step_split(int dbl, int L, int* L1, int* L2) {
+// The split for an axis whose columns reach ein rows on the input and eout on
+// the output (n1 < L1 <= ein, k2 < L2 <= eout).  fast: the most balanced one
+// whose L2 has the two-radix first pass (four_step_first) and whose L1 is
+// compiled; without one (or for other sides) as described above.
+static bool four_step_split(int dbl, int L, bool fast, long long ein, long long eout, int* L1, int* L2) {
+  if (fast) {
+    int best_m = 0;
+    for (int m = 2; m <= 1024 && m < L; ++m) {
+      if (L % m != 0 || !find_four_step_kernel(dbl, m)) continue;
+      const int c = L / m;
+      if (c > ein || m > eout || four_step_factor(dbl, c) != VARIANT_DIRECT) continue;
+      if (!best_m || std::max(m, c) < std::max(best_m, L / best_m)) best_m = m;
+    }
+    if (best_m) {
+      *L1 = L / best_m;
+      *L2 = best_m;
+      return true;
+    }
+  }
   int best = 0, best_static = 0;
   for (int d = 2; (long long)d * d <= L; ++d) {
     if (L % d != 0) continue;
@@ -1239,51 +1288,117 @@ static bool four_step_split(int dbl, int L, int* L1, int* L2) {
       best_static = st;
     }
   }
-  if (!best) return false;
+  if (!best || best > ein || L / best > eout) return false;
   *L1 = best;
   *L2 = L / best;
   return true;
 }
 
+// Does four_step_first serve the first pass of this axis (plain complex
+// input, with Bluestein's chirp or filter, unit inner stride)?
+static bool four_step_fast(const PassSpec& s) {
+  return s.I == 1 && s.in.kind == IO_CPLX && s.in.si == 1 && s.in.sk == 1;
+}
+
+static Pass make_four_step_first(const PassSpec& s, int L1, const FourStepKernel* k, const void* twl) {
+  Pass p;
+  p.fsfirst = true;
+  p.is_static = true;
+  p.fn = k->fn;
+  PassDesc& d = p.d;  // for describe()
+  d.L = k->M;
+  d.nst = 2;
+  d.radix[0] = k->r0;
+  d.radix[1] = k->r1;
+  d.P = k->P;
+  d.C = k->cs;
+  d.I = 1;
+  d.Q = (long long)L1 * s.O;
+  d.inverse = s.inverse;
+  FourStepGeom& g = p.fsgeom;
+  g.L1 = L1;
+  g.tiles = (L1 + k->cs - 1) / k->cs;
+  g.in_o = s.in.so;
+  g.out_o = (long long)L1 * k->M;
+  g.chirp = s.in.chirp;
+  g.mul = s.in.mul;
+  g.chirp_n = s.in.chirp_n;
+  g.inverse = s.inverse;
+  auto tw = twiddle_table(s.dbl, k->M, 1, 0, k->M, false);
+  g.tw = tw->p;
+  g.twl = twl;
+  p.tables.push_back(tw);
+  for (auto& t : s.keep) p.tables.push_back(t);
+  const long long nblk = (long long)g.tiles * s.O;
+  if (nblk > 0x7fffffffLL) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "too many columns for one launch"};
+  p.grid = dim3((unsigned)nblk);
+  p.block = dim3((unsigned)(k->cs * k->P));
+  p.smem = k->smem;
+  cuda_check(ensure_smem_attr(p.fn, p.smem), "cudaFuncSetAttribute(four-step)");
+  return p;
+}
+
+// W_L^m for m < kTwSplit, then W_L^(kTwSplit m) for kTwSplit m < L
+// (conjugated for an inverse).
+static std::shared_ptr<DevTable> split_twiddles(int dbl, long long L, bool conj) {
+  const int hi = (int)((L + kTwSplit - 1) / kTwSplit);
+  const size_t esz = dbl ? 16 : 8;
+  auto lo_t = twiddle_table(dbl, L, 1, 0, kTwSplit, conj);
+  auto hi_t = twiddle_table(dbl, L, kTwSplit, 0, hi, conj);
+  auto t = std::make_shared<DevTable>();
+  cuda_check(cudaGetDevice(&t->device), "cudaGetDevice");
+  t->bytes = esz * (size_t)(kTwSplit + hi);
+  cuda_check(cudaMalloc(&t->p, t->bytes), "cudaMalloc(four-step twiddles)");
+  cuda_check(cudaMemcpy(t->p, lo_t->p, esz * kTwSplit, cudaMemcpyDeviceToDevice), "cudaMemcpy(four-step twiddles)");
+  cuda_check(cudaMemcpy(static_cast<char*>(t->p) + esz * kTwSplit, hi_t->p, esz * hi, cudaMemcpyDeviceToDevice),
+             "cudaMemcpy(four-step twiddles)");
+  // device-to-device copies do not wait: the first execute may be on a stream of its own
+  cuda_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize(four-step twiddles)");
+  return t;
+}
+
 // The pass pair of a four-step transform of length s.L = L1 * L2 along a
 // complex axis with unit inner stride (element (i, n, o) at i + n I + o so).
 // Pass A reads s.in (its chirp / mul indexed along the whole axis) and
-// writes the scratch (I, L, O) times the twiddle; pass B reads the scratch
-// and writes s.out at k2 + L2 k1 (with its chirp and the scale).
-static void four_step_pair(const PassSpec& s, int L1, int L2, Pass* pa, Pass* pb) {
+// writes the scratch (I, L2, L1, O); pass B reads the scratch and writes
+// s.out in order (with its chirp and the scale).
+static void four_step_pair(const PassSpec& s, int L1, int L2, unsigned flags, Pass* pa, Pass* pb) {
   const long long L = (long long)L1 * L2;
-  auto tw = twiddle_table(s.dbl, L, 1, 0, (int)L, s.inverse != 0);
+  auto tw = split_twiddles(s.dbl, L, s.inverse != 0);
   PassSpec a = s;
   a.L = L2;
-  a.I = s.I * L1;
-  a.O = s.O;
+  a.I = s.I;
+  a.O = L1 * s.O;
   a.scale = 1.0;
   a.fast_io = false;
   a.epi = false;
   a.C = 0;
   a.variant = four_step_factor(s.dbl, L2);
-  a.in.sk = s.I * L1;  // si = 1 and so as for the whole axis
+  // columns (i, n1) at i + n1 I, then o
+  a.in.sk = s.I * L1;
+  a.in.so = s.I;
+  a.in.o1 = L1;
+  a.in.so2 = s.in.so;
   // sub-axis index j from the column base b = i + j I + o so: (b mod so) / I
-  // (so need not be a multiple of I L1: Bluestein's input has L < L1 L2 rows)
   if (a.in.chirp || a.in.mul || a.in.kind == IO_HERM_FULL || a.in.kind == IO_R2R) {
     a.in.t_i = s.I;
-    a.in.t_ia = a.in.so;
+    a.in.t_ia = s.in.so;
     a.in.t_m = L1;
   }
   a.out = IoAny{};
   a.out.kind = IO_CPLX_TW;
   a.out.si = 1;
-  a.out.so = s.I * L;
-  a.out.sk = s.I * L1;
+  a.out.so = s.I * L2;
+  a.out.sk = s.I;
   a.out.w = tw->p;
   a.out.n = (int)L;
-  a.out.t_i = s.I;
+  a.out.t_i = s.I * L2;
   a.out.t_ia = s.I * L;
   a.keep.push_back(tw);
   PassSpec b = s;
   b.L = L1;
-  b.I = s.I;
-  b.O = (long long)L2 * s.O;
+  b.I = s.I * L2;
+  b.O = s.O;
   b.fast_io = s.out.kind == IO_CPLX && !s.out.chirp;
   b.epi = false;
   b.C = 0;
@@ -1291,19 +1406,37 @@ static void four_step_pair(const PassSpec& s, int L1, int L2, Pass* pa, Pass* pb
   b.in = IoAny{};
   b.in.kind = IO_CPLX;
   b.in.si = 1;
-  b.in.so = s.I * L1;
-  b.in.sk = s.I;
+  b.in.so = s.I * L;
+  b.in.sk = s.I * L2;
   b.out.sk = s.I * L2;
-  b.out.so = s.I;
-  b.out.o1 = L2;
-  b.out.so2 = s.out.so;
   if (b.out.chirp || b.out.kind == IO_TRUNC || b.out.kind == IO_R2R) {
     b.out.t_i = s.I;
     b.out.t_ia = s.out.so;
     b.out.t_m = L2;
   }
-  *pa = make_pass(a);
-  *pb = make_pass(b);
+  const FourStepKernel* fk = four_step_fast(s) ? find_four_step_kernel(s.dbl, L2) : nullptr;
+  if (fk) {
+    PassSpec f = s;
+    f.keep.push_back(tw);
+    *pa = make_four_step_first(f, L1, fk, tw->p);
+  } else {
+    *pa = make_pass(a);
+  }
+  if (b.fast_io) {
+    const StaticPlan* sp = find_static(s.dbl, L1);
+    b.variant = pipe_strided_ok(b, sp, s.dbl ? 16 : 8) ? VARIANT_PIPE : VARIANT_AUTO;
+    try {
+      *pb = b.variant == VARIANT_PIPE ? make_pass(b) : plan_pass(b, flags);
+    } catch (const Error& e) {
+      if (b.variant != VARIANT_PIPE) throw;
+      b.variant = VARIANT_AUTO;
+      *pb = plan_pass(b, flags);
+    }
+  } else {
+    *pb = make_pass(b);
+  }
+  pa->four_step = 1;
+  pb->four_step = 2;
 }
 
 static bool plain_complex_axis(const PassSpec& s) {
@@ -1346,125 +1479,10 @@ static bool four_step_extents(const PassSpec& s, long long* ein, long long* eout
   return true;
 }
 
-// Axis swap pass (i, a, b, o) -> (i, b, a, o) over an I x A x B x O array.
-static Pass make_swap_pass(int dbl, long long I, long long A, long long B, long long O) {
-  Pass p;
-  p.swap = true;
-  p.swg = SwapGeom{I, A, B, O};
-  p.d.L = 1;
-  p.d.I = I;
-  p.d.Q = I * A * B * O;
-  p.fn = swap_axes_kernel(dbl, I == 1);
-  p.block = dim3(256);
-  const long long units = I == 1 ? ((A + 31) / 32) * ((B + 31) / 32) * O : (A * B * O + 7) / 8;
-  long long nb = (long long)sm_count() * 8;
-  if (nb > units) nb = units;
-  p.grid = dim3((unsigned)(nb > 0 ? nb : 1));
-  return p;
-}
-
-// The fast form of a plain complex four-step axis, three passes through one
-// scratch (the strided and contiguous passes keep their pipelined kernels):
-//   1. L2-point transforms along n2 (columns (i, n1), stride I L1) with the
-//      twiddle W_L^(n1 k2) applied to the transformed tile before its store;
-//   2. L1-point transforms along n1 (columns (i) per (k2, o), stride I), in
-//      place, leaving (i, k1, k2);
-//   3. the swap of the k1 and k2 axes into the output: (i, k2, k1), i.e.
-//      index k2 + L2 k1 along the axis.
-// Needs the pipelined strided kernel for L2 (else false, nothing added).
-// fast_split picks the largest strided factor with such a kernel (so the
-// contiguous factor is as short as it can be) whose cofactor is a length
-// one pass handles.
-static bool fast_split(int dbl, int L, int* Lc, int* Ls) {
-  for (int d = dbl ? 512 : 1024; d >= 2; --d) {
-    if (L % d != 0) continue;
-    const StaticPlan* sp = find_static(dbl, d);
-    if (!sp || !sp->pipe_s || sp->P > sp->lb) continue;
-    const int c = L / d;
-    // (a contiguous factor beyond one static plan runs the one-column
-    // dynamic kernel, slower than the two-pass form: 2^24 ComplexF32 1.28
-    // against 0.73 ms)
-    if (c < 2 || !four_step_factor(dbl, c)) continue;
-    *Ls = d;
-    *Lc = c;
-    return true;
-  }
-  return false;
-}
-
-static bool add_four_step_fast(std::vector<Pass>& out, const PassSpec& s, unsigned flags, int L1, int L2,
-                               int src, int dst) {
-  const long long L = (long long)L1 * L2;
-  PassSpec a;
-  a.dbl = s.dbl;
-  a.L = L2;
-  a.I = s.I * L1;
-  a.O = s.O;
-  a.inverse = s.inverse;
-  a.scale = 1.0;
-  a.in = s.in;
-  a.in.sk = s.I * L1;  // si = 1 and so = I L as for the whole axis
-  a.out = IoAny{};
-  a.out.kind = IO_CPLX;
-  a.out.si = 1;
-  a.out.sk = s.I * L1;
-  a.out.so = s.I * L;
-  a.fast_io = true;
-  a.variant = VARIANT_PIPE;
-  Pass pa;
-  try {
-    pa = make_pass(a);
-  } catch (const Error& e) {
-    if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE && e.status != DFFT_ERROR_INVALID_VALUE) throw;
-    return false;
-  }
-  if (!pa.tma || !pa.pipe) return false;  // the hook lives in the strided pipelined kernel
-  // W_L^m = W_L^(m mod B) * W_L^(B * (m / B)), two small tables
-  const int Bt = 1024;
-  auto lo = twiddle_table(s.dbl, L, 1, 0, Bt, s.inverse != 0);
-  auto hi = twiddle_table(s.dbl, L, Bt, 0, (int)((L + Bt - 1) / Bt), s.inverse != 0);
-  pa.tables.push_back(lo);
-  pa.tables.push_back(hi);
-  pa.geom.tw_lo = lo->p;
-  pa.geom.tw_hi = hi->p;
-  pa.geom.tw_div = s.I;
-  pa.geom.tw_lf = L;
-  pa.geom.tw_b = Bt;
-  PassSpec b;
-  b.dbl = s.dbl;
-  b.L = L1;
-  b.I = s.I;
-  b.O = (long long)L2 * s.O;
-  b.inverse = s.inverse;
-  b.scale = s.scale;
-  b.in.kind = b.out.kind = IO_CPLX;
-  b.in.si = b.out.si = 1;
-  b.in.sk = b.out.sk = s.I;
-  b.in.so = b.out.so = s.I * L1;
-  b.fast_io = true;
-  Pass pb;
-  try {
-    pb = plan_pass(b, flags);
-  } catch (const Error& e) {
-    if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
-    return false;
-  }
-  Pass pc = make_swap_pass(s.dbl, s.I, L1, L2, s.O);
-  pa.src = src;
-  pa.dst = BUF_CHIRP;
-  pb.src = BUF_CHIRP;
-  pb.dst = BUF_CHIRP;
-  pc.src = BUF_CHIRP;
-  pc.dst = dst;
-  out.push_back(std::move(pa));
-  out.push_back(std::move(pb));
-  out.push_back(std::move(pc));
-  return true;
-}
-
-static size_t add_four_step(std::vector<Pass>& out, const PassSpec& s, int L1, int L2, int src, int dst) {
+static size_t add_four_step(std::vector<Pass>& out, const PassSpec& s, unsigned flags, int L1, int L2, int src,
+                            int dst) {
   Pass pa, pb;
-  four_step_pair(s, L1, L2, &pa, &pb);
+  four_step_pair(s, L1, L2, flags, &pa, &pb);
   pa.src = src;
   pa.dst = BUF_CHIRP;
   pb.src = BUF_CHIRP;
@@ -1487,10 +1505,10 @@ static size_t add_direct_passes(std::vector<Pass>& out, const PassSpec& s, unsig
     if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
   }
   int L1 = 0, L2 = 0;
-  if (!plain_complex_axis(s) || !four_step_split(s.dbl, s.L, &L1, &L2))
+  if (!plain_complex_axis(s) || !four_step_split(s.dbl, s.L, four_step_fast(s), s.L, s.L, &L1, &L2))
     throw Error{DFFT_ERROR_UNSUPPORTED_SIZE,
                 "length " + std::to_string(s.L) + " has no single-pass or four-step form"};
-  return add_four_step(out, s, L1, L2, src, dst);
+  return add_four_step(out, s, flags, L1, L2, src, dst);
 }
 
 // ---------------------------------------------------------------------------
@@ -1527,23 +1545,11 @@ static std::shared_ptr<DevTable> upload(int dbl, const std::vector<long double>&
   return t;
 }
 
-// Convolution length for an N-point axis: of the 5-smooth lengths up to a
-// third above the smallest, the one with the least work (length x stages) in
-// a compiled kernel; the smallest one where none is compiled.
+// Convolution length for an N-point axis: the shortest compiled one, else the
+// smallest 5-smooth one.
 static int bluestein_length(int dbl, int N) {
-  const int least = smooth5_at_least(2 * N - 1);
-  int best = least;
-  long long cost = -1;
-  for (long long m = least; m <= least + least / 3LL && m <= (1 << 14); ++m) {
-    const StaticPlan* sp = find_static(dbl, (int)m);
-    if (!sp || sp->P > sp->lb) continue;
-    const long long c = m * (sp->nst + 2);
-    if (cost < 0 || c < cost) {
-      cost = c;
-      best = (int)m;
-    }
-  }
-  return best;
+  if (const ChirpAnyKernel* k = find_chirp_any(dbl, 2 * N - 1)) return k->L;
+  return smooth5_at_least(2 * N - 1);
 }
 
 struct BluesteinTables {
@@ -1677,15 +1683,8 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   {
     long long ein = 0, eout = 0;
     int L1 = 0, L2 = 0;
-    if (four_step_extents(s, &ein, &eout) && four_step_split(s.dbl, L, &L1, &L2) && L1 <= ein && L2 <= eout) {
-      // plain complex sides: the three-pass form (strided pass on a factor
-      // with a pipelined kernel, contiguous pass on its cofactor)
-      int Lc = 0, Ls = 0;
-      if (plain_complex_axis(s) && fast_split(s.dbl, L, &Lc, &Ls) &&
-          add_four_step_fast(out, s, flags, Lc, Ls, src, dst))
-        return (size_t)(s.I * s.O) * (size_t)L * (s.dbl ? 16 : 8);
-      return add_four_step(out, s, L1, L2, src, dst);
-    }
+    if (four_step_extents(s, &ein, &eout) && four_step_split(s.dbl, L, four_step_fast(s), ein, eout, &L1, &L2))
+      return add_four_step(out, s, flags, L1, L2, src, dst);
   }
   if (L > (1 << 23)) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "length too large for Bluestein"};
   // complex sides up to 512 (ComplexF32) / 256 points (ComplexF64): two-radix
@@ -1702,7 +1701,19 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   }
   // the outer direction is in the tables; the inner FFT_M pair is forward
   // then inverse
-  const int M = bluestein_length(s.dbl, L);
+  int M = bluestein_length(s.dbl, L);
+  if (four_step_fast(s) && !find_chirp_any(s.dbl, 2 * L - 1)) {
+    // convolutions beyond one CTA: the smallest length that splits into the
+    // two-radix first pass and a compiled factor of at most 2048 (1000003
+    // ComplexF32 points: 109 us through 1024 x 2000, 174 us through 1350 x
+    // 1500, the smallest one)
+    for (int m = M, i = 0; i < 64 && m < M + M / 4; m = smooth5_at_least(m + 1), ++i) {
+      int m1 = 0, m2 = 0;
+      if (!four_step_split(s.dbl, m, true, L, L, &m1, &m2) || !find_four_step_kernel(s.dbl, m2) || m1 > 2048) continue;
+      M = m;
+      break;
+    }
+  }
   const BluesteinTables bt = bluestein_tables(s.dbl, L, s.inverse ? +1 : -1, M);
   const size_t csz = s.dbl ? 16 : 8;
   // both FFT_M, the filter and the two chirp multiplies on one tile in
@@ -1772,11 +1783,11 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   // the sub-axis index of a column must stay inside the column's extent
   // on both sides (n1 < M1 rows of the input, k2 < M2 rows of the output)
   long long ein = 0, eout = 0;
-  if (!four_step_extents(s, &ein, &eout) || !four_step_split(s.dbl, M, &M1, &M2) || M2 > eout || M1 > ein)
+  if (!four_step_extents(s, &ein, &eout) || !four_step_split(s.dbl, M, four_step_fast(s), ein, eout, &M1, &M2))
     throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "length " + std::to_string(L) + " is too long for Bluestein here"};
   Pass p[4];
-  four_step_pair(a, M1, M2, &p[0], &p[1]);
-  four_step_pair(b, M1, M2, &p[2], &p[3]);
+  four_step_pair(a, M1, M2, flags, &p[0], &p[1]);
+  four_step_pair(b, M1, M2, flags, &p[2], &p[3]);
   p[0].src = src;
   p[0].dst = BUF_CHIRP;
   p[1].src = BUF_CHIRP;

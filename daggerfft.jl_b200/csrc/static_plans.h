@@ -12,7 +12,7 @@ struct StaticPlan {
   int radix[8];       // stage radices
   int lb;             // __launch_bounds__ of the kernels (max threads per CTA)
   const void* fast;   // axis_pass_static: complex in, complex out
-  const void* any;    // axis_pass_any: any IoKind, R2C post-pass, one-launch Bluestein
+  const void* any;    // axis_pass_any: any IoKind, R2C post-pass
   const void* pipe_s; // axis_pass_pipe<T, LB, false, ...>: strided C2C, TMA-pipelined (or null)
   const void* pipe_c; // axis_pass_pipe<T, LB, true, ...>: contiguous C2C, bulk-copy pipelined
   int pipe_lb;        // __launch_bounds__ of the pipelined kernels

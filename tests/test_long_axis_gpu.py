@@ -171,3 +171,31 @@ def test_long_axis_fast_form(dtype, shape, dims):
     assert rel(to_np(F), oracle.fft(a, dims=dims)) <= tol
     _, B = _run(dfft.IFFT(), F, dims)
     assert rel(to_np(B), a) <= tol
+
+
+@pytest.mark.parametrize("m,c", [(128, 143), (160, 143), (192, 91), (225, 91), (240, 91), (256, 143), (320, 169),
+                                 (360, 91), (384, 343), (480, 343), (512, 343), (576, 343), (768, 539), (1024, 539)])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_two_radix_first_pass(m, c, dtype):
+    # every compiled length of the first pass (columns c not a multiple of the
+    # tile), two transforms, forward and inverse
+    a = rand((m * c, 2), dtype, seed=m)
+    p, F = _run(dfft.FFT(), to_gpu(a), (1,))
+    first = p.describe().splitlines()[0]
+    assert first.startswith(f"four-step-first L={m} "), first
+    tol = tol_for(dtype)
+    assert rel(to_np(F), oracle.fft(a, dims=(1,))) <= tol
+    _, B = _run(dfft.IFFT(), F, (1,))
+    assert rel(to_np(B), a) <= tol
+
+
+@pytest.mark.parametrize("n", [20011, 1000003])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_prime_over_two_radix_first_pass(n, dtype):
+    # Bluestein's chirp and filter on the first passes' loads
+    a = rand((n, 3), dtype, seed=n % 89)
+    p, F = _run(dfft.FFT(), to_gpu(a), (1,))
+    assert p.describe().count("four-step-first") == 2, p.describe()
+    assert rel(to_np(F), oracle.fft(a, dims=(1,))) <= tol_for(dtype)
+    _, B = _run(dfft.IFFT(), F, (1,))
+    assert rel(to_np(B), a) <= tol_for(dtype)
