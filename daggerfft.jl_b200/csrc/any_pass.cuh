@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(LB, 1) axis_pass_any(const __grid_constant__ P
   const int t = d.cfast ? tid / d.C : tid % P;
   const PadCol<V> col{sm + (size_t)c * d.ld};
   const GlobalTw<V> tw{reinterpret_cast<const V*>(d.tw)};
+  pass_entry();
   tile_load<T>(d, sm, L);
   __syncthreads();
   static_stages<T, L, P, 1, 0, 1, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(d, t, col, col, col,
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(1024) axis_pass_dynamic(const __grid_constant_
   const int c = d.cfast ? tid % d.C : tid / P;
   const int t = d.cfast ? tid / d.C : tid % P;
   V* col = sm + (size_t)c * d.ld;
+  pass_entry();
   tile_load<T>(d, sm, L);
   __syncthreads();
   for (int half = 0;; ++half) {

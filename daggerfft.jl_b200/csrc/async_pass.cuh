@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(LB, MINB) axis_pass_async(const PassDesc d, co
     const V* gtw = reinterpret_cast<const V*>(d.tw);
     for (int i = tid; i < g.ntw; i += LB) stw[i] = gtw[i];
   }
+  pass_entry();
   const V* src = reinterpret_cast<const V*>(d.in.p);
   // thread tid copies column c = tid % CS, rows t, t + LB/CS, ... of a tile
   // (LB is a multiple of CS): element e = tid + i*LB of the [row][column]

@@ -114,6 +114,19 @@ template <typename V> __device__ __forceinline__ int swz(int k) {
 
 template <typename V> __device__ __forceinline__ V ldg_c(const V* p) { return __ldg(p); }
 
+// Every pass kernel calls this before its first access to the arrays, from
+// all threads: it waits until the kernels before it in the stream are
+// complete and visible, then lets the next one be scheduled.  The passes of
+// a transform are launched with programmatic stream serialization, so the
+// next pass's launch and set-up overlap this one's tail instead of following
+// it (a kernel launched without that attribute does not wait here).  Tables
+// that never change may be read earlier; arrays another pass writes are read
+// with plain loads, not through the read-only path, since that pass may still
+// be running when this kernel starts.
+__device__ __forceinline__ void pass_entry() {
+  asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Element access for every side kind.  The r2r maps (FFTW kinds, all
 // unnormalised) express each kind as one complex FFT:
@@ -416,6 +429,7 @@ __global__ void __launch_bounds__(LB) axis_pass_static(const PassDesc d) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* sm = reinterpret_cast<V*>(smem_raw);
   const ColCtx x = col_ctx(d, P);
+  pass_entry();
   const PadCol<V> col{sm + x.c * d.ld};
   const GlobalTw<V> tw{reinterpret_cast<const V*>(d.tw)};
   static_stages<T, L, P, 0, 0, 0, 1, 1, 0, PadCol<V>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(

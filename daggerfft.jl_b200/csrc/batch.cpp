@@ -89,7 +89,7 @@ static void capture(Batch* B, const void* const* ins, void* const* outs, cudaGra
         for (int j = 0; j < i; ++j)
           if (B->plans[j] == B->plans[i]) { branch[i] = branch[j]; break; }
     }
-    for (int i = 0; i < n; ++i) execute_plan(B->plans[i], ins[i], outs[i], B->side[branch[i]]);
+    for (int i = 0; i < n; ++i) execute_plan(B->plans[i], ins[i], outs[i], B->side[branch[i]], nullptr, nullptr, false);
     for (int i = 0; i < k; ++i) {
       cuda_check(cudaEventRecord(B->join[i], B->side[i]), "cudaEventRecord(join)");
       cuda_check(cudaStreamWaitEvent(s, B->join[i], 0), "cudaStreamWaitEvent(join)");

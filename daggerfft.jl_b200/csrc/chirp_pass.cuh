@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(CS* P, MINB) axis_pass_chirp(const __grid_cons
   const long long qo = !cv ? 0 : d.I == 1 ? q : q / d.I;
   const long long qi = !cv || d.I == 1 ? 0 : q - qo * d.I;
 
+  pass_entry();
   {  // radix R0 of the padded input
     const V* in = reinterpret_cast<const V*>(d.in.p) + (qi * d.in.si + io_outer(d.in, qo));
     const long long sk = d.in.sk;

@@ -47,6 +47,7 @@ struct Pass {
   int src = BUF_IN, dst = BUF_OUT;
   size_t src_off = 0, dst_off = 0;  // byte offsets into those buffers
   bool is_static = false;
+  int dbl = 0;  // precision
   int four_step = 0;  // 1, 2: first / second pass of a four-step axis
   bool fsfirst = false;  // four_step_first
   FourStepGeom fsgeom{};
@@ -215,7 +216,9 @@ int wisdom_size();
 
 // Launches one pass on `stream` with the given buffers; `work` holds the
 // counters of a fused slab pass (p.ctr_bytes, zeroed here before the launch).
-cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream, void* work = nullptr);
+// overlap: the launch may overlap the tail of the kernel before it.
+cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream, void* work = nullptr,
+                        bool overlap = true);
 
 // Raise the dynamic shared-memory limit of a kernel on the current device.
 cudaError_t ensure_smem_attr(const void* fn, size_t bytes);

@@ -38,8 +38,9 @@ Plan* build_slab_split_plan(int precision, int inverse, int64_t L, int64_t nslab
 
 // work / chirp: workspaces supplied by the caller for this execution (null:
 // the plan's own); a plan built with kFlagCallerWorkspace owns none.
+// overlap: the launches may overlap the tails of the kernels before them.
 void execute_plan(const Plan* p, const void* in, void* out, cudaStream_t stream, void* work = nullptr,
-                  void* chirp = nullptr);
+                  void* chirp = nullptr, bool overlap = true);
 
 // Internal plan flag (above the public DFFT_FLAG_* bits): allocate no
 // workspace; every execution brings its own (the serving runtime's arena).

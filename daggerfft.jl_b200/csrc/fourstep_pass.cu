@@ -19,8 +19,8 @@ namespace dfft {
   X(double, 1, 2, 2, 24, 32, 24) X(double, 1, 2, 2, 32, 32, 32)
 
 #define INST(T, DBL, MINB, CS, P, R0, R1)                                                                   \
-  template __global__ void four_step_first<T, MINB, CS, P, R0, R1>(const cvec<T>::type* __restrict__,       \
-                                                                   cvec<T>::type* __restrict__,             \
+  template __global__ void four_step_first<T, MINB, CS, P, R0, R1>(const cvec<T>::type*,                    \
+                                                                   cvec<T>::type*,                          \
                                                                    const __grid_constant__ FourStepGeom);
 DFFT_FS(INST)
 #undef INST

@@ -46,7 +46,7 @@ template <typename V, int CS, int R0, int R1> struct FourStepTile {
 
 template <typename T, int MINB, int CS, int P, int R0, int R1>
 __global__ void __launch_bounds__(CS* P, MINB)
-    four_step_first(const typename cvec<T>::type* __restrict__ in, typename cvec<T>::type* __restrict__ out,
+    four_step_first(const typename cvec<T>::type* in, typename cvec<T>::type* out,
                     const __grid_constant__ FourStepGeom g) {
   typedef typename cvec<T>::type V;
   typedef FourStepTile<V, CS, R0, R1> Tile;
@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(CS* P, MINB)
   const int n1_0 = (blockIdx.x - o * g.tiles) * CS;
   const V* twl = reinterpret_cast<const V*>(g.twl);
   const V* tw = reinterpret_cast<const V*>(g.tw);
+  for (int i = tid; i < kTwSplit; i += CS * P) lo[i] = twl[i];
+  pass_entry();
   {
     const int c = tid % CS, j = tid / CS;
     const int n1 = n1_0 + c;
@@ -72,7 +74,6 @@ __global__ void __launch_bounds__(CS* P, MINB)
       v[r] = mk<V>((T)0, (T)0);
       if (n1 < g.L1 && (!g.chirp || n1 + n < g.chirp_n)) v[r] = src[n];
     }
-    for (int i = tid; i < kTwSplit; i += CS * P) lo[i] = twl[i];
     if (g.chirp || g.mul) {
       const V* f = reinterpret_cast<const V*>(g.chirp ? g.chirp : g.mul) + n1;
 #pragma unroll

@@ -337,6 +337,7 @@ static Pass make_feed_pass(const PassSpec& s) {
   if (!s.inverse && s.scale != 1.0) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "scaled forward strided pass"};
   const std::vector<int> rad(k->radix, k->radix + k->nst);
   Pass p;
+  p.dbl = s.dbl;
   p.feed = true;
   p.is_static = true;
   p.fn = s.inverse ? k->fn_inv : k->fn;
@@ -417,6 +418,7 @@ static Pass make_async_pass(const PassSpec& s) {
   if (!s.inverse && s.scale != 1.0) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "scaled forward strided pass"};
   const std::vector<int> rad(k->radix, k->radix + k->nst);
   Pass p;
+  p.dbl = s.dbl;
   p.async_ = true;
   p.is_static = true;
   p.fn = s.inverse ? k->fn_inv : k->fn;
@@ -490,6 +492,7 @@ static Pass make_real_pass(const PassSpec& s) {
   if (s.O % k->cs != 0) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "pencils do not split into whole tiles"};
   const std::vector<int> rad(k->radix, k->radix + k->nst);
   Pass p;
+  p.dbl = s.dbl;
   p.real = true;
   p.is_static = true;
   p.fn = kind == 1 ? k->fn : k->fn_inv;
@@ -577,6 +580,7 @@ static Pass make_tiled_pass(const PassSpec& s) {
   const int n = s.in.n;
   const int C = k->cs;
   Pass p;
+  p.dbl = s.dbl;
   p.tiled = kind;
   p.tdbl = s.dbl;
   p.is_static = true;
@@ -668,6 +672,7 @@ Pass make_pass(const PassSpec& s) {
     }
   }
   Pass p;
+  p.dbl = s.dbl;
   PassDesc& d = p.d;
   const int L = s.L;
   if (L < 1) throw Error{DFFT_ERROR_INVALID_VALUE, "transform length must be >= 1"};
@@ -690,13 +695,20 @@ Pass make_pass(const PassSpec& s) {
   }
   int variant = s.variant;
   if (variant == VARIANT_AUTO) {
-    // strided axes: the producer-fed kernel for passes of 16 MiB and more
-    // (below that its persistent grid is not filled and the one-tile kernels
-    // are as fast), unless rows lie 1 MiB or more apart (each tile then
-    // touches L pages, and the narrower tile rows of that kernel pay the
-    // address translation twice as often)
-    if (feed_ok(s, esz) && s.I * (long long)esz < (1LL << 20) &&
-        (double)s.I * (double)s.O * (double)L * esz >= (double)(16 << 20)) {
+    // Short passes run the one-tile kernel: its direct loads start sooner than
+    // a TMA pipeline, CTAs are handed out as SMs free up, and they overlap the
+    // pass before (us, TMA kernel against one-tile: 96^3 ComplexF32 10.9 /
+    // 4.9, 120 x 160 x 80 axis 3 11.7 / 6.8, 96^3 ComplexF64 12.9 / 6.3).
+    // ComplexF32: strided axes up to 16 MiB; above, the producer-fed kernel
+    // moves more (64 uneven grids: the larger ones fed 922 us, one-tile up to
+    // 48 MB 1006; contiguous axes too 950).  ComplexF64: every axis while both
+    // sides fit L2 (128^3 fft + ifft 73 us, with TMA kernels 80).
+    const double side = (double)s.I * (double)s.O * (double)L * esz;
+    const bool small = sp && side <= (s.dbl ? 48e6 : s.I > 1 ? (double)(16 << 20) : 0.0);
+    // strided axes: the producer-fed kernel, unless rows lie 1 MiB or more
+    // apart (each tile then touches L pages, and the narrower tile rows of
+    // that kernel pay the address translation twice as often)
+    if (!small && feed_ok(s, esz) && s.I * (long long)esz < (1LL << 20)) {
       // the first (fastest) default launch shape whose tile width fits I
       for (int v = 0; const SlabKernel* k = find_strided_kernel(s.dbl, L, v); ++v) {
         if (!k->dflt || k->cs > s.I) continue;
@@ -711,8 +723,7 @@ Pass make_pass(const PassSpec& s) {
       }
     }
     // the same passes with rows TMA cannot address: cp.async tiles
-    if (!feed_ok(s, esz) && (s.I * (long long)esz) % 16 != 0 && async_ok(s, esz) &&
-        (double)s.I * (double)s.O * (double)L * esz >= (double)(16 << 20)) {
+    if (!small && !feed_ok(s, esz) && (s.I * (long long)esz) % 16 != 0 && async_ok(s, esz)) {
       for (int v = 0; const SlabKernel* k = find_async_kernel(s.dbl, L, v); ++v) {
         if (!k->dflt || k->cs > s.I) continue;
         PassSpec t = s;
@@ -725,7 +736,7 @@ Pass make_pass(const PassSpec& s) {
         break;
       }
     }
-    if (pipe_strided_ok(s, sp, esz) || pipe_contig_ok(s, sp, esz)) {
+    if (!small && (pipe_strided_ok(s, sp, esz) || pipe_contig_ok(s, sp, esz))) {
       PassSpec t = s;
       t.variant = VARIANT_PIPE;
       try {
@@ -819,7 +830,9 @@ Pass make_pass(const PassSpec& s) {
       C = sp->pipe_cs;
     } else if (C <= 0) {
       C = 1;
-      while (C * 2 * P <= 256 && smem_for(C * 2) <= smax) C *= 2;
+      // (at least three CTAs per SM: 16384 pencils of 128 points 12.9 -> 10.8
+      // us ComplexF32, 17.0 -> 14.9 ComplexF64, against one CTA of 256 threads)
+      while (C * 2 * P <= 256 && smem_for(C * 2) <= smax / 3) C *= 2;
     }
     while (C > 1 && (C * P > lb || smem_for(C) > smax)) C /= 2;
     if (!contig && C % 2) C = 2;  // 16-byte TMA rows for complex float
@@ -874,16 +887,15 @@ Pass make_pass(const PassSpec& s) {
   int C = s.C;
   if (C <= 0) {
     if (d.cfast) {
-      // rows of at least 128 bytes for coalesced strided loads, ~256 threads
+      // rows of 128 bytes for coalesced strided loads, more only to fill two
+      // warps (120 x 160 x 80 ComplexF32 axis 3: 16 columns 6.8 us, 32 8.0).
+      // A CTA's loads, stages and stores follow one another, so several CTAs
+      // per SM rather than one of 1024 threads keep the memory busy, and short
+      // passes get two per SM, while rows still fill sectors (2^20 ComplexF32:
+      // 128 CTAs of 8 columns against 256 of 4).
       C = s.dbl ? 8 : 16;
-      while (C * P < 256 && C < 64) C *= 2;
-      // the kernels that stage the whole tile have their loads, stages and
-      // stores one after another: several CTAs per SM, not one of 1024
-      // threads, keep the memory busy (rows of 64 bytes still fill sectors)
-      // and short passes get two CTAs per SM while rows fill a sector (2^20
-      // ComplexF32: 128 CTAs of 8 columns against 256 of 4)
-      if (!s.fast_io)
-        while ((C * P > 512 && C * esz > 64) || (C * esz > 32 && (Q + C - 1) / C < 2 * sm_count())) C /= 2;
+      while (C * P < 64 && C < 64) C *= 2;
+      while ((C * P > 512 && C * esz > 64) || (C * esz > 32 && (Q + C - 1) / C < 2 * sm_count())) C /= 2;
     } else {
       C = 1;
       while (C * 2 * P <= 256) C *= 2;
@@ -935,6 +947,7 @@ Pass make_slab_pass(int dbl, int L, long long O, int inverse, int v) {
   const int esz = dbl ? 16 : 8;
   const std::vector<int> rad(k->radix, k->radix + k->nst);
   Pass p;
+  p.dbl = dbl;
   p.slab = true;
   p.is_static = true;
   p.fn = inverse ? k->fn_inv : k->fn;
@@ -1097,7 +1110,33 @@ Pass make_slab_split_pass(int dbl, int L, long long nslab, int inverse, int v, i
   return p;
 }
 
-cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream, void* work) {
+// Launch that may overlap its predecessor's tail (programmatic stream
+// serialization; the kernel waits for it in pass_entry()).  Passes over up to
+// 96 MB gain one launch latency each (128^3 ComplexF64 fft + ifft, 6 passes of
+// 67 MB: 86 -> 75 us).  Longer ones are launched in the ordinary way: their
+// persistent CTAs would be placed between the predecessor's last ones, and
+// where those leave shared memory in pieces an SM ends up with fewer of them
+// for the whole pass (256^3 Float64 rfft: 166 -> 196 us).  So are the
+// transforms of a batch, which overlap one another already (64 uneven grids:
+// 1086 against 1095 us), the slab pass, which follows a memset, and the mixed
+// pass, which does not call pass_entry().
+static cudaError_t launch_serial(const Pass& p, void** args, cudaStream_t stream, bool overlap) {
+  const double bytes = 2.0 * (double)p.d.L * (double)p.d.Q * (p.dbl ? 16 : 8);
+  if (!overlap || bytes > 96e6) return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = p.grid;
+  cfg.blockDim = p.block;
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, p.fn, args);
+}
+
+cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream, void* work, bool overlap) {
   if (p.grid.x == 0) return cudaSuccess;
   cudaError_t e = ensure_smem_attr(p.fn, p.smem);
   if (e != cudaSuccess) return e;
@@ -1138,14 +1177,14 @@ cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream,
     g.src = in;
     g.dst = out;
     void* args[] = {&d, &tin, &tout, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   if (p.real) {
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15)
       return cudaErrorMisalignedAddress;
     RealGeom g = p.rgeom;
     void* args[] = {&d, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   if (p.async_) {
     // the cp.async kernels move 8-byte (ComplexF32) elements
@@ -1153,7 +1192,7 @@ cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream,
       return cudaErrorMisalignedAddress;
     AsyncGeom g = p.ageom;
     void* args[] = {&d, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   if (p.feed) {
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15)
@@ -1167,14 +1206,14 @@ cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream,
     if (e != cudaSuccess) return e;
     StridedGeom g = p.fgeom;
     void* args[] = {&d, &tin, &tout, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   if (p.fsfirst) {
     const void* ip = in;
     void* op = out;
     FourStepGeom g = p.fsgeom;
     void* args[] = {&ip, &op, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   if (p.slab) {
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15)
@@ -1216,10 +1255,10 @@ cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream,
     }
     TmaGeom g = p.geom;
     void* args[] = {&d, &tin, &tout, &g};
-    return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+    return launch_serial(p, args, stream, overlap);
   }
   void* args[] = {&d};
-  return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, stream);
+  return launch_serial(p, args, stream, overlap);
 }
 
 }  // namespace dfft
@@ -1302,6 +1341,7 @@ static bool four_step_fast(const PassSpec& s) {
 
 static Pass make_four_step_first(const PassSpec& s, int L1, const FourStepKernel* k, const void* twl) {
   Pass p;
+  p.dbl = s.dbl;
   p.fsfirst = true;
   p.is_static = true;
   p.fn = k->fn;
@@ -1638,6 +1678,7 @@ static Pass make_chirp_pass(const PassSpec& s, const ChirpKernel* k) {
   const int M = k->M;
   const BluesteinTables bt = bluestein_tables(s.dbl, s.L, s.inverse ? +1 : -1, M);
   Pass p;
+  p.dbl = s.dbl;
   p.is_static = true;
   p.fn = s.I > 1 ? k->fn : k->fn_contig;
   PassDesc& d = p.d;

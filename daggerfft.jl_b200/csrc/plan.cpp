@@ -384,7 +384,8 @@ Plan::~Plan() {
 size_t Plan::in_bytes() const { return (size_t)(in_shape[0] * in_shape[1] * in_shape[2]) * in_elem; }
 size_t Plan::out_bytes() const { return (size_t)(out_shape[0] * out_shape[1] * out_shape[2]) * out_elem; }
 
-void execute_plan(const Plan* P, const void* in, void* out, cudaStream_t stream, void* work, void* chirp) {
+void execute_plan(const Plan* P, const void* in, void* out, cudaStream_t stream, void* work, void* chirp,
+                  bool overlap) {
   if (!in || !out) throw Error{DFFT_ERROR_INVALID_VALUE, "in/out is NULL"};
   if (!work) work = P->work;
   if (!chirp) chirp = P->chirp;
@@ -401,7 +402,7 @@ void execute_plan(const Plan* P, const void* in, void* out, cudaStream_t stream,
     if (err != cudaSuccess) break;
     void* bufs[4] = {const_cast<void*>(in), out, work, chirp};
     err = launch_pass(p, static_cast<char*>(bufs[p.src]) + p.src_off, static_cast<char*>(bufs[p.dst]) + p.dst_off,
-                      stream, work);
+                      stream, work, overlap);
   }
   if (cur != P->device) cudaSetDevice(cur);
   cuda_check(err, "kernel launch");

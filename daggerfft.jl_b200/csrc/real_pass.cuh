@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
     for (int i = tid; i <= M; i += blockDim.x) sw[i] = gw[i];
   }
   __syncthreads();
+  pass_entry();
 
   if (tid >= NC) {
     if (tid == NC) {

@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(LB, MINB)
   const V* gtw = reinterpret_cast<const V*>(dx.tw);
   for (int i = tid; i < g.ntw; i += blockDim.x) stw[i] = gtw[i];
   __syncthreads();
+  pass_entry();
 
   if (tid >= NC) {
     if (tid == NC) {
@@ -471,6 +472,7 @@ __global__ void __launch_bounds__(LB, MINB)
   const V* gtw = reinterpret_cast<const V*>(d.tw);
   for (int i = tid; i < g.ntw; i += blockDim.x) stw[i] = gtw[i];
   __syncthreads();
+  pass_entry();
 
   if (tid >= NC) {
     if (tid == NC) {

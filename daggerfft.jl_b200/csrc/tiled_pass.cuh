@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(LB, MINB)
     }
   }
   __syncthreads();
+  pass_entry();
 
   if (tid >= NC) {
     if (tid == NC) {

@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(LB) axis_pass_pipe(const PassDesc d,
   const V* gtw = reinterpret_cast<const V*>(d.tw);
   for (int i = tid; i < g.ntw; i += blockDim.x) stw[i] = gtw[i];
   __syncthreads();
+  pass_entry();
   if (s_abort) return;  // misaligned layout: nothing was issued
   const int C = g.C;
   const StageTw<V> tw{stw};
