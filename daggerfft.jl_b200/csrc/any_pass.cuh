@@ -350,10 +350,10 @@ __device__ __noinline__ void dyn_stage(const PassDesc& d, int s, int t, typename
   const int ns = d.ns[s], ts = d.tws[s];
   if constexpr (CTW) {
     const ComputedTw<V> g{d.L};
-    stage_body<T, R, EMAX / R, 1, 0, 1>(d, d.L, d.P, ns, ts, 0, s == 0, s == d.nst - 1, t, c, c, g, 0, 0, true);
+    stage_body<T, R, EMAX / R, 1, 0, 1, false>(d, d.L, d.P, ns, ts, 0, s == 0, s == d.nst - 1, t, c, c, g, 0, 0, true);
   } else {
     const GlobalTw<V> g{reinterpret_cast<const V*>(d.tw)};
-    stage_body<T, R, EMAX / R, 1, 0, 1>(d, d.L, d.P, ns, ts, 0, s == 0, s == d.nst - 1, t, c, c, g, 0, 0, true);
+    stage_body<T, R, EMAX / R, 1, 0, 1, false>(d, d.L, d.P, ns, ts, 0, s == 0, s == d.nst - 1, t, c, c, g, 0, 0, true);
   }
 }
 

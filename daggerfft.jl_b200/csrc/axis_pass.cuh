@@ -296,7 +296,14 @@ template <int BAR> __device__ __forceinline__ void stage_sync() {
 // CIN/COUT: the shared-memory views the stage reads and writes (they differ
 // when a stage moves a tile between a dense TMA buffer and a padded one).
 // toff: offset of this stage in a StageTw table (Ns - R_0).
-template <typename T, int R, int BMAX, int SMEM_IO, int BAR, int DIR, class CIN, class COUT, class TW>
+// CLAMP (static radices on a tile in shared memory): a thread past the last
+// butterfly computes that one again and stores nothing.  Butterflies behind a
+// condition, even one that always holds (t < P is not visible to the compiler
+// when the mapping is chosen at run time), spilled in the kernels that loop
+// over tiles: the 12 x 16 slab pass 300 bytes a thread, and 2^20 ComplexF32
+// points 39 instead of 30 us through the pipelined pass.  The kernels that
+// load and store memory directly hold fewer registers with the condition.
+template <typename T, int R, int BMAX, int SMEM_IO, int BAR, int DIR, bool CLAMP, class CIN, class COUT, class TW>
 __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int Ns, int ts, int toff,
                                            bool first, bool last, int t, const CIN& cin,
                                            const COUT& cout, const TW& tw, long long ib,
@@ -312,11 +319,12 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
   const T scale = DIR == 1 || fold ? (T)1 : (T)d.scale;
   const bool to_global = SMEM_IO != 1 && last;
   const bool from_global = SMEM_IO == 0 && first;
+  const bool exact = CLAMP && BMAX * P == Lr;
   V v[BMAX][R];
 #pragma unroll
   for (int b = 0; b < BMAX; ++b) {
-    const int j = t + b * P;
-    if (j < Lr) {
+    const int j = CLAMP && !exact ? min(t + b * P, Lr - 1) : t + b * P;
+    if (CLAMP || j < Lr) {
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int k = j + r * Lr;
@@ -337,8 +345,9 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
   if (!from_global) stage_sync<BAR>();
 #pragma unroll
   for (int b = 0; b < BMAX; ++b) {
-    const int j = t + b * P;
-    if (j < Lr) {
+    const int j = CLAMP && !exact ? min(t + b * P, Lr - 1) : t + b * P;
+    const bool mine = exact || t + b * P < Lr;
+    if (CLAMP || j < Lr) {
       const int jm = j % Ns;
       if (!first) {
 #pragma unroll
@@ -351,7 +360,7 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
       for (int r = 0; r < R; ++r) {
         const int k = o0 + r * Ns;
         if (to_global) {
-          if (cv) {
+          if (cv && mine) {
             V y = v[b][r];
             if (inv) y.y = -y.y;
             // SMEM_IO 2 (the fused slab pass) stores whole pencils: unit stride;
@@ -361,9 +370,9 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
         } else if (SMEM_IO == 1 && last) {
           V y = v[b][r];
           if (inv) y.y = -y.y;
-          cout.st(o0, r * Ns, cscale(y, scale));
+          if (mine) cout.st(o0, r * Ns, cscale(y, scale));
         } else {
-          cout.st(o0, r * Ns, v[b][r]);
+          if (mine) cout.st(o0, r * Ns, v[b][r]);
         }
       }
     }
@@ -410,13 +419,13 @@ __device__ __forceinline__ void static_stages(const PassDesc& d, int t, const CF
   constexpr bool LAST = (sizeof...(Rest) == 0);
   constexpr int R0_ = FIRST ? R : R0;
   if constexpr (FIRST && LAST) {
-    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, true, t, cf, cl, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR, SMEM_IO != 0>(d, L, P, NS, TS, NS - R0_, true, true, t, cf, cl, tw, ib, ob, cv);
   } else if constexpr (FIRST) {
-    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, true, false, t, cf, cm, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR, SMEM_IO != 0>(d, L, P, NS, TS, NS - R0_, true, false, t, cf, cm, tw, ib, ob, cv);
   } else if constexpr (LAST) {
-    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, true, t, cm, cl, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR, SMEM_IO != 0>(d, L, P, NS, TS, NS - R0_, false, true, t, cm, cl, tw, ib, ob, cv);
   } else {
-    stage_body<T, R, BM, SMEM_IO, BAR, DIR>(d, L, P, NS, TS, NS - R0_, false, false, t, cm, cm, tw, ib, ob, cv);
+    stage_body<T, R, BM, SMEM_IO, BAR, DIR, SMEM_IO != 0>(d, L, P, NS, TS, NS - R0_, false, false, t, cm, cm, tw, ib, ob, cv);
   }
   if constexpr (sizeof...(Rest) > 0)
     static_stages<T, L, P, SMEM_IO, BAR, DIR, NS * R, R0_, S + 1, CFIRST, CMID, CLAST, TW, Rest...>(

@@ -94,7 +94,7 @@ struct SlabKernel {
   int lb;   // threads per CTA
   int cs;   // pencils / columns per tile
   int nb;   // tile buffers
-  int dflt; // an untuned plan may pick this variant
+  int dflt; // an untuned plan may pick this variant (2, fused slab: for arrays of 48 MB and more)
   const void* fn;      // forward
   const void* fn_inv;  // inverse
   const void* fn_split;      // forward, rows split by rank

@@ -54,6 +54,18 @@ DFFT_SLAB_INST(double, 96, 5, 2, 256, 16, 4, 16, 16)
 DFFT_SLAB_INST(double, 96, 6, 2, 256, 16, 4, 16, 16)
 DFFT_SLAB_INST(double, 96, 3, 3, 256, 16, 4, 16, 16)
 
+// 384 = 24 x 16 and 192 = 12 x 16, plain layout only
+#define DFFT_SLAB_INST2(T, LB, MINB, NB, L, P, CS, ...)             \
+  DFFT_SLAB_INST1(T, LB, MINB, NB, 1, 0, L, P, CS, __VA_ARGS__)      \
+  DFFT_SLAB_INST1(T, LB, MINB, NB, 2, 0, L, P, CS, __VA_ARGS__)
+#define K2(T, LB, MINB, NB, L, P, CS, ...)                                       \
+  (const void*)&slab_xy_pass<T, LB, MINB, NB, 1, 0, L, P, CS, __VA_ARGS__>,     \
+      (const void*)&slab_xy_pass<T, LB, MINB, NB, 2, 0, L, P, CS, __VA_ARGS__>, nullptr, nullptr, nullptr, nullptr
+DFFT_SLAB_INST2(float, 160, 4, 2, 384, 16, 8, 24, 16)
+DFFT_SLAB_INST2(float, 160, 6, 2, 192, 16, 8, 12, 16)
+DFFT_SLAB_INST2(double, 96, 4, 2, 384, 16, 4, 24, 16)
+DFFT_SLAB_INST2(double, 96, 6, 2, 192, 16, 4, 12, 16)
+
 // Variants of one (precision, L) are listed fastest first (B200, 512^3 /
 // 256^3 / 128^3 arrays); `dflt` marks the ones an untuned plan may use (at
 // L = 128 the per-axis passes are faster, so only DFFT_FLAG_TUNE or
@@ -72,6 +84,10 @@ static const SlabKernel kSlabKernels[] = {
     {0, 256, 16, 2, {16, 16}, 288, 16, 3, 1, K(float, 288, 2, 3, 256, 16, 16, 16, 16)},
     {0, 128, 8, 2, {16, 8}, 160, 16, 2, 0, K(float, 160, 6, 2, 128, 8, 16, 16, 8)},
     {0, 128, 8, 2, {16, 8}, 160, 16, 3, 0, K(float, 160, 4, 3, 128, 8, 16, 16, 8)},
+    {0, 384, 16, 2, {24, 16}, 160, 8, 2, 2, K2(float, 160, 4, 2, 384, 16, 8, 24, 16)},
+    {0, 192, 16, 2, {12, 16}, 160, 8, 2, 2, K2(float, 160, 6, 2, 192, 16, 8, 12, 16)},
+    {1, 384, 16, 2, {24, 16}, 96, 4, 2, 2, K2(double, 96, 4, 2, 384, 16, 4, 24, 16)},
+    {1, 192, 16, 2, {12, 16}, 96, 4, 2, 2, K2(double, 96, 6, 2, 192, 16, 4, 12, 16)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 2, 1, K(double, 160, 5, 2, 512, 64, 2, 8, 8, 8)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 2, 1, K(double, 160, 4, 2, 512, 64, 2, 8, 8, 8)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 3, 1, K(double, 160, 3, 3, 512, 64, 2, 8, 8, 8)},
@@ -81,6 +97,7 @@ static const SlabKernel kSlabKernels[] = {
 };
 
 #undef K
+#undef K2
 
 const SlabKernel* find_slab_kernel(int dbl, int L, int v) {
   int i = 0;

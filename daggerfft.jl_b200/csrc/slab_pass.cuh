@@ -129,6 +129,35 @@ template <typename V, int CS, int R0> struct YSwzCol {
 };
 template <int R, int... Rest> struct first_radix { static constexpr int value = R; };
 
+// The same for two-radix lengths that are not powers of two (384 = 24 x 16,
+// 192 = 12 x 16: dims 1 and 2 of 384^3 ComplexF32 374 us as two passes, 228
+// fused; of 192^3 ComplexF64 93 and 78).  Element k = R0 q + s: the first stage's butterfly j writes
+// (q = j, s = r), the second's reads (q = r, s = j), so one of the two is a
+// constant in every access.  s is XORed with m(q) < g, g the power of two in
+// R0 up to the slots of 128 bytes: it stays inside its aligned group of g
+// (g divides R0), and consecutive q, R0 slots apart, fall on different ones.
+__host__ __device__ constexpr int pow2_part(int r, int most) {
+  int g = 1;
+  while (g < most && r % (2 * g) == 0) g *= 2;
+  return g;
+}
+template <int SLOTS, int R0> __device__ __forceinline__ int two_swz(int q, int s) {
+  constexpr int g = pow2_part(R0, SLOTS);
+  return R0 * q + (s & ~(g - 1)) + ((s & (g - 1)) ^ ((q / (SLOTS / g)) & (g - 1)));
+}
+template <typename V, int L, int R0> struct XTwoCol {
+  V* p;  // the pencil's dense start
+  static constexpr int SLOTS = 128 / (int)sizeof(V);
+  __device__ __forceinline__ V ld(int b, int off) const { return p[two_swz<SLOTS, R0>(off / R0, b)]; }
+  __device__ __forceinline__ void st(int b, int off, V v) const { p[two_swz<SLOTS, R0>(b / R0, off)] = v; }
+};
+template <typename V, int CS, int R0> struct YTwoCol {
+  V* p;  // the tile buffer + column
+  static constexpr int SLOTS = 128 / (int)sizeof(V) > CS ? 128 / (int)sizeof(V) / CS : 1;  // rows per 128 bytes
+  __device__ __forceinline__ V ld(int b, int off) const { return p[two_swz<SLOTS, R0>(off / R0, b) * CS]; }
+  __device__ __forceinline__ void st(int b, int off, V v) const { p[two_swz<SLOTS, R0>(b / R0, off) * CS] = v; }
+};
+
 // Tile buffer of CS pencils written in pieces of 2^rsh elements: element k
 // of pencil c at ((k >> rsh) * CS + c) * 2^rsh + (k mod 2^rsh), so piece s of
 // all CS pencils is one contiguous run (one bulk store per rank block).
@@ -187,6 +216,11 @@ __global__ void __launch_bounds__(LB, MINB)
   constexpr int NC = CS * P;  // stage threads
   static_assert(NC % 32 == 0 && NC + 32 == LB, "whole warps of stage threads plus one producer warp");
   static_assert(NB >= 2 && NB <= 4, "tile buffers");
+  constexpr int R0 = first_radix<Rs...>::value;
+  constexpr bool kPow2 = (L & (L - 1)) == 0;
+  static_assert(kPow2 || (sizeof...(Rs) == 2 && MODE == 0), "other lengths: two radices, plain layout");
+  typedef typename std::conditional<kPow2, XSwzCol<V, L, R0>, XTwoCol<V, L, R0>>::type XMid;
+  typedef typename std::conditional<kPow2, YSwzCol<V, CS, R0>, YTwoCol<V, CS, R0>>::type YMid;
   extern __shared__ __align__(128) unsigned char smem_slab[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_slab);
   uint64_t* empty = reinterpret_cast<uint64_t*>(smem_slab + 32);
@@ -370,7 +404,6 @@ __global__ void __launch_bounds__(LB, MINB)
     // phases scale by 1/L)
     typedef typename std::conditional<DIR == 2, StageTwScaledLast<V>, StageTw<V>>::type TWT;
     const TWT tw{stw};
-    constexpr int R0 = first_radix<Rs...>::value;
     for (int it = 0;; ++it) {
       const int b = it % NB;
       if (!mbar_wait_bounded(&full[b], (uint32_t)((it / NB) & 1))) s_cabort = 1;
@@ -384,21 +417,23 @@ __global__ void __launch_bounds__(LB, MINB)
         // (the producer bulk-stores the tile)
         const int t = tid % P, c = tid / P;
         const StrideCol<V> dense{buf + (size_t)c * L, 1};
-        const XSwzCol<V, L, R0> sw{buf + (size_t)c * L, c};
+        XMid sw;
+        sw.p = buf + (size_t)c * L;
+        if constexpr (kPow2) sw.c = c;
         if constexpr (YX) {
           // out in pieces of rout elements, piece s of every pencil together
           const PieceCol<V> pc{buf, c, CS, __ffs(g.rout) - 1};
-          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, PieceCol<V>,
+          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XMid, PieceCol<V>,
                         TWT, Rs...>(dx, t, dense, sw, pc, tw, 0, 0, true);
         } else {
-          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XSwzCol<V, L, R0>, StrideCol<V>,
+          static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideCol<V>, XMid, StrideCol<V>,
                         TWT, Rs...>(dx, t, dense, sw, dense, tw, 0, 0, true);
         }
       } else {
         const int c = tid % CS, t = tid / CS;
         const StrideColC<V, CS> dense{buf + c};
-        const YSwzCol<V, CS, R0> sw{buf + c};
-        static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YSwzCol<V, CS, R0>, StrideColC<V, CS>,
+        const YMid sw{buf + c};
+        static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, StrideColC<V, CS>, YMid, StrideColC<V, CS>,
                       TWT, Rs...>(dy, t, dense, sw, dense, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the buffer is next read (store) or written (load) by TMA

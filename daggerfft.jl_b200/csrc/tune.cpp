@@ -195,7 +195,9 @@ int choose_slab(int dbl, int L, long long O, int inverse, const std::vector<Pass
   std::vector<int> idx;
   const bool tune = (flags & DFFT_FLAG_TUNE) != 0;
   for (int v = 0; const SlabKernel* k = find_slab_kernel(dbl, L, v); ++v) {
-    if (!tune && !k->dflt && !(flags & DFFT_FLAG_FUSE)) continue;
+    // (an L2-resident array gains nothing from the single sweep of memory)
+    const bool dflt = k->dflt == 1 || (k->dflt == 2 && (double)L * L * (double)O * (dbl ? 16 : 8) >= 48e6);
+    if (!tune && !dflt && !(flags & DFFT_FLAG_FUSE)) continue;
     try {
       cands.push_back(make_slab_pass(dbl, L, O, inverse, v));
       idx.push_back(v);

@@ -175,3 +175,23 @@ def test_every_fused_variant(dtype, L, inverse, tmp_path):
         assert rel(to_np(y), ref) <= tol_for(dtype), (v, d)
     if (dtype, L) == (np.complex64, 512):
         assert radices == {"8x8x8", "32x16"}
+
+
+@pytest.mark.parametrize("L,O", [(192, 1), (192, 5), (384, 2)])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_two_radix_lengths(L, O, dtype):
+    # 192 = 12 x 16 and 384 = 24 x 16 (radix counts that do not divide the
+    # threads per pencil), forward, inverse and in place
+    a = rand((L, L, O), dtype, seed=L + O)
+    g = to_gpu(a)
+    tol = tol_for(dtype)
+    ref = oracle.fft(a, dims=(1, 2))
+    p = dfft.gpu_plan_transform(dfft.FFT(), g, (1, 2), flags=dfft.FLAG_FUSE)
+    assert p.launches == 1 and p.describe().startswith("slab-xy"), p.describe()
+    out = dfft.empty_like_layout(p.out_shape, g.dtype, g)
+    p.execute(g, out)
+    assert rel(to_np(out), ref) <= tol
+    q = dfft.gpu_plan_transform(dfft.IFFT_(), out, (1, 2), flags=dfft.FLAG_FUSE)
+    q.execute(out, out)
+    assert rel(to_np(out), a) <= tol
+    assert dfft.device_error() == 0
