@@ -33,15 +33,22 @@ struct Choice {
 std::mutex g_w_mu;
 std::map<std::string, Choice> g_wisdom;
 
+// (cudaGetDeviceProperties takes a millisecond or more, once per pass of
+// every plan: kept per device)
 std::string device_tag() {
+  static std::mutex mu;
+  static std::map<int, std::string> tags;
   int dev = 0;
   cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = tags.find(dev);
+  if (it != tags.end()) return it->second;
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return "unknown";
   std::string n(prop.name);
   for (char& c : n)
     if (c == ' ' || c == '|') c = '_';
-  return n + "_sm" + std::to_string(prop.multiProcessorCount);
+  return tags[dev] = n + "_sm" + std::to_string(prop.multiProcessorCount);
 }
 
 std::string key_of(const PassSpec& s) {

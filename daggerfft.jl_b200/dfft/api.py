@@ -84,6 +84,7 @@ FFT_ = _tag("FFT!", _lib.T_FFT_INPLACE)
 IFFT_ = _tag("IFFT!", _lib.T_IFFT_INPLACE)
 RFFT_ = _tag("RFFT!", _lib.T_RFFT_INPLACE)
 IRFFT_ = _tag("IRFFT!", _lib.T_IRFFT_INPLACE)
+_FFT, _IFFT, _RFFT, _IRFFT = FFT(), IFFT(), RFFT(), IRFFT()
 
 # FFTW r2r kinds (fftw_r2r_kind values)
 R2HC, HC2R, DHT = 0, 1, 2
@@ -128,6 +129,14 @@ def _order(t: torch.Tensor) -> str:
         return "F"
     if t.is_contiguous():
         return "C"
+    step = 1
+    for n, st in zip(t.shape, t.stride()):
+        if st != step:
+            break
+        step *= n
+    else:
+        return "F"
+    # (extents of 1 leave their strides free)
     if t.permute(*reversed(range(t.dim()))).is_contiguous():
         return "F"
     return "X"
@@ -144,6 +153,26 @@ def empty_like_layout(shape, dtype, like: torch.Tensor):
     """A new tensor of ``shape``/``dtype`` in the memory order of ``like``."""
     o = _order(like)
     return _empty(shape, dtype, like.device, "F" if o == "F" else "C")
+
+
+def _strides(shape, order):
+    """Element strides of a dense array of ``shape`` in memory order ``order``."""
+    st, step = [0] * len(shape), 1
+    for i in (range(len(shape)) if order == "F" else reversed(range(len(shape)))):
+        st[i] = step
+        step *= max(shape[i], 1)
+    return tuple(st)
+
+
+# the current stream's handle without a Stream object (about 1 us of the
+# 18 us a small transform's call took)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _stream_handle(device_index):
+    if _raw_stream is not None:
+        return _raw_stream(device_index)
+    return torch.cuda.current_stream(device_index).cuda_stream
 
 
 def _norm_dims(dims, ndim) -> Tuple[int, ...]:
@@ -217,6 +246,7 @@ class Plan:
         wb = ctypes.c_size_t()
         check(L.dfft_plan_workspace_bytes(h, ctypes.byref(wb)))
         self.workspace_bytes = wb.value
+        self._out_strides = _strides(self.out_shape, order)
 
     def describe(self) -> str:
         """One line per kernel launch (kernel kind, length, columns, launch
@@ -227,10 +257,12 @@ class Plan:
 
     def execute(self, inp: torch.Tensor, out: torch.Tensor, stream=None):
         if stream is None:
-            stream = torch.cuda.current_stream(inp.device)
-        s = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream or 0)
-        check(self._L.dfft_execute(self._h, ctypes.c_void_p(inp.data_ptr()),
-                                   ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(s)))
+            s = _stream_handle(inp.device.index)
+        else:
+            s = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream or 0)
+        st = self._L.dfft_execute(self._h, inp.data_ptr(), out.data_ptr(), s)
+        if st:
+            check(st)
         return out
 
     def __del__(self):
@@ -250,7 +282,10 @@ _CACHE_LOCK = threading.Lock()
 def gpu_plan_transform(transform, A: torch.Tensor, dims, n=None, decomp=None, method="plain",
                        flags=0) -> Plan:
     """src/fftgpu.jl:85-105: a fresh plan for tag ``transform`` on ``A``."""
-    o = _order(A)
+    return _new_plan(transform, A, _order(A), dims, n, decomp, method, flags)
+
+
+def _new_plan(transform, A, o, dims, n, decomp, method, flags):
     if o == "X":
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, "array must be contiguous (C or Fortran order)")
     return Plan(transform, tuple(A.shape), A.dtype, dims, order=o, n=n, decomp=decomp,
@@ -263,16 +298,18 @@ def get_or_create_gpu_plan(transform, A: torch.Tensor, dims, n=None, decomp=None
     device, real length, decomposition and arithmetic form."""
     if not isinstance(transform, Transform):
         raise ArgumentError(_lib.ERROR_UNKNOWN_TRANSFORM, "Unknown transform type")
+    return _cached_plan(transform, A, _order(A), dims, n, decomp, method, flags)
+
+
+def _cached_plan(transform, A, o, dims, n, decomp, method, flags):
     dims_t = tuple(dims) if isinstance(dims, (tuple, list)) else (int(dims),)
-    key = (A.dtype, tuple(A.shape), _order(A), transform, dims_t, n, type(decomp or Pencil()),
+    key = (A.dtype, tuple(A.shape), o, transform, dims_t, n, Pencil if decomp is None else type(decomp),
            method, flags, A.device.index)
-    with _CACHE_LOCK:
-        p = GPU_PLAN_CACHE.get(key)
+    p = GPU_PLAN_CACHE.get(key)
     if p is None:
-        p = gpu_plan_transform(transform, A, dims_t, n, decomp, method, flags)
+        p = _new_plan(transform, A, o, dims_t, n, decomp, method, flags)
         with _CACHE_LOCK:
-            GPU_PLAN_CACHE.setdefault(key, p)
-            p = GPU_PLAN_CACHE[key]
+            p = GPU_PLAN_CACHE.setdefault(key, p)
     return p
 
 
@@ -312,9 +349,12 @@ def _prep(A):
 
 
 def _run(transform, A, dims, n=None, decomp=None, method="plain", flags=0, out_dtype=None):
-    A = _prep(A)
-    p = get_or_create_gpu_plan(transform, A, dims, n, decomp, method, flags)
-    out = empty_like_layout(p.out_shape, out_dtype or A.dtype, A)
+    _check_tensor(A)
+    o = _order(A)
+    if o == "X":
+        A, o = A.contiguous(), "C"
+    p = _cached_plan(transform, A, o, dims, n, decomp, method, flags)
+    out = torch.empty_strided(p.out_shape, p._out_strides, dtype=out_dtype or A.dtype, device=A.device)
     return p.execute(A, out)
 
 
@@ -349,7 +389,7 @@ def fft(A, decomp=None, dims=(1, 2, 3), transforms=None, method="plain"):
         return _run(r, A, dims, decomp=decomp)
     if not A.is_complex():
         A = A.to(_complex_dtype(A.dtype))
-    return _run(FFT(), A, dims, decomp=decomp, method=method)
+    return _run(_FFT, A, dims, decomp=decomp, method=method)
 
 
 def ifft(A, decomp=None, dims=(1, 2, 3), transforms=None, method="plain"):
@@ -363,7 +403,7 @@ def ifft(A, decomp=None, dims=(1, 2, 3), transforms=None, method="plain"):
         return _run(r, A, dims, decomp=decomp)
     if not A.is_complex():
         A = A.to(_complex_dtype(A.dtype))
-    return _run(IFFT(), A, dims, decomp=decomp, method=method)
+    return _run(_IFFT, A, dims, decomp=decomp, method=method)
 
 
 def rfft(A, decomp=None, dims=(1, 2, 3)):
@@ -371,7 +411,7 @@ def rfft(A, decomp=None, dims=(1, 2, 3)):
     dims = _norm_dims(dims, A.dim())
     if A.is_complex():
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, "rfft takes a real array")
-    return _run(RFFT(), A, dims, decomp=decomp, out_dtype=_complex_dtype(A.dtype))
+    return _run(_RFFT, A, dims, decomp=decomp, out_dtype=_complex_dtype(A.dtype))
 
 
 def irfft(F, d, decomp=None, dims=(1, 2, 3), destroy_input=False):
@@ -380,7 +420,7 @@ def irfft(F, d, decomp=None, dims=(1, 2, 3), destroy_input=False):
     if not F.is_complex():
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, "irfft takes a complex array")
     flags = _lib.FLAG_DESTROY_INPUT if destroy_input else 0
-    return _run(IRFFT(), F, dims, n=int(d), decomp=decomp, flags=flags,
+    return _run(_IRFFT, F, dims, n=int(d), decomp=decomp, flags=flags,
                 out_dtype=_real_dtype(F.dtype))
 
 
