@@ -112,7 +112,7 @@ const SlabKernel* find_async_kernel(int dbl, int L, int v = 0);
 const SlabKernel* find_real_kernel(int dbl, int M);
 // A compiled tiled_pass (tiled_pass.cu).
 struct TiledKernel {
-  int dbl, L, P, nst, radix[4];
+  int dbl, L, P, nst, radix[4];  // L: real length, radices of L/2
   int lb;       // threads per CTA
   int cs;       // pencils / columns per tile
   int strided;  // 0 contiguous axis, 1 strided axis

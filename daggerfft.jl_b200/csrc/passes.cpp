@@ -573,9 +573,9 @@ static int tiled_kind(const PassSpec& s) {
 
 static Pass make_tiled_pass(const PassSpec& s) {
   const int kind = tiled_kind(s);
-  const int L = s.L;
+  const int L = s.L / 2;  // FFT of the N reals packed in pairs
   const int rsz = s.dbl ? 8 : 4, csz = 2 * rsz;
-  const TiledKernel* k = kind ? find_tiled_kernel(s.dbl, L, kind == 2 ? 1 : 0, s.in.r2r) : nullptr;
+  const TiledKernel* k = kind ? find_tiled_kernel(s.dbl, s.L, kind == 2 ? 1 : 0, s.in.r2r) : nullptr;
   if (!k) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "no tiled kernel for this pass"};
   const int n = s.in.n;
   const int C = k->cs;
@@ -586,7 +586,6 @@ static Pass make_tiled_pass(const PassSpec& s) {
   p.is_static = true;
   p.fn = k->fn;
   TiledGeom& g = p.tgeom;
-  g.n_in = g.n_out = n;
   if (kind == 1) {
     if (s.O % C != 0 || ((size_t)C * n * rsz) % 16 != 0)
       throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "pencils do not split into whole tiles"};
@@ -637,8 +636,12 @@ static Pass make_tiled_pass(const PassSpec& s) {
   auto tw = twiddle_table(s.dbl, L, 1, 0, L, false);
   p.tables.push_back(tw);
   d.tw = tw->p;
+  auto w = twiddle_table(s.dbl, n, 1, 0, L + 1, false);
+  p.tables.push_back(w);
+  d.tw2 = w->p;
   g.ld = ld;
-  g.bstride = (int)(((size_t)C * n * rsz + 127) & ~(size_t)127);
+  // (contiguous tiles: pencils 64 bytes further apart than their length)
+  g.bstride = (int)(((size_t)C * (n + (kind == 1 ? 64 / rsz : 0)) * rsz + 127) & ~(size_t)127);
   g.err = device_error_word();
   p.smem = kSlabHeader + 2 * (size_t)g.bstride + (size_t)C * ld * csz;
   p.block = dim3((unsigned)k->lb);
@@ -701,10 +704,10 @@ Pass make_pass(const PassSpec& s) {
     // 4.9, 120 x 160 x 80 axis 3 11.7 / 6.8, 96^3 ComplexF64 12.9 / 6.3).
     // ComplexF32: strided axes up to 16 MiB; above, the producer-fed kernel
     // moves more (64 uneven grids: the larger ones fed 922 us, one-tile up to
-    // 48 MB 1006; contiguous axes too 950).  ComplexF64: every axis while both
+    // 48 MB 1006; contiguous axes too 950), contiguous ones up to 4 MB.  ComplexF64: every axis while both
     // sides fit L2 (128^3 fft + ifft 73 us, with TMA kernels 80).
     const double side = (double)s.I * (double)s.O * (double)L * esz;
-    const bool small = sp && side <= (s.dbl ? 48e6 : s.I > 1 ? (double)(16 << 20) : 0.0);
+    const bool small = sp && side <= (s.dbl ? 48e6 : s.I > 1 ? (double)(16 << 20) : 4e6);
     // strided axes: the producer-fed kernel, unless rows lie 1 MiB or more
     // apart (each tile then touches L pages, and the narrower tile rows of
     // that kernel pay the address translation twice as often)
@@ -895,7 +898,9 @@ Pass make_pass(const PassSpec& s) {
       // 128 CTAs of 8 columns against 256 of 4).
       C = s.dbl ? 8 : 16;
       while (C * P < 64 && C < 64) C *= 2;
-      while ((C * P > 512 && C * esz > 64) || (C * esz > 32 && (Q + C - 1) / C < 2 * sm_count())) C /= 2;
+      while ((C * P > 512 && C * esz > 64) ||
+             (C * P > 64 && C * esz > 32 && (Q + C - 1) / C < 2 * sm_count()))
+        C /= 2;
     } else {
       C = 1;
       while (C * 2 * P <= 256) C *= 2;

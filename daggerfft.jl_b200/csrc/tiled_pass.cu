@@ -1,7 +1,8 @@
 // Instantiations of the tile-staged R2R pass (tiled_pass) for DCT-II and
-// DCT-III: FFT lengths 128, 256, 512, contiguous (whole pencils) and strided
-// (column tiles) axes.  threads = C*P stage threads + one producer warp;
-// two tile buffers.
+// DCT-III: N = 128, 256, 512 (FFTs of N/2), contiguous (whole pencils) and
+// strided (column tiles) axes.  threads = C*P stage threads + one producer
+// warp; two tile buffers; small tiles, so that 32 planes of 256 x 256 are
+// under two per CTA.
 #include "dfft_internal.h"
 
 namespace dfft {
@@ -16,39 +17,38 @@ namespace dfft {
 #define K(T, LB, MINB, S, KIND, L, P, C, ...) (const void*)&tiled_pass<T, LB, MINB, 2, S, KIND, L, P, C, __VA_ARGS__>
 
 // kinds 5 = REDFT10 (DCT-II), 4 = REDFT01 (DCT-III)
-DFFT_TILED_BOTH(double, 160, 3, 0, 128, 8, 16, 16, 8)
-DFFT_TILED_BOTH(double, 160, 3, 1, 128, 8, 16, 16, 8)
-DFFT_TILED_BOTH(double, 160, 3, 0, 256, 16, 8, 16, 16)
-DFFT_TILED_BOTH(double, 160, 3, 1, 256, 16, 8, 16, 16)
-DFFT_TILED_BOTH(double, 160, 3, 0, 512, 64, 2, 8, 8, 8)
-DFFT_TILED_BOTH(double, 288, 2, 1, 512, 64, 4, 8, 8, 8)
-DFFT_TILED_BOTH(float, 160, 3, 0, 128, 8, 16, 16, 8)
-DFFT_TILED_BOTH(float, 160, 3, 1, 128, 8, 16, 16, 8)
-DFFT_TILED_BOTH(float, 160, 3, 0, 256, 16, 8, 16, 16)
-DFFT_TILED_BOTH(float, 288, 2, 1, 256, 16, 16, 16, 16)
-DFFT_TILED_BOTH(float, 160, 3, 0, 512, 64, 2, 8, 8, 8)
-DFFT_TILED_BOTH(float, 288, 2, 1, 512, 64, 4, 8, 8, 8)
+DFFT_TILED_BOTH(double, 96, 4, 0, 128, 8, 8, 8, 8)
+DFFT_TILED_BOTH(double, 96, 4, 1, 128, 8, 8, 8, 8)
+DFFT_TILED_BOTH(double, 96, 4, 0, 256, 8, 8, 16, 8)
+DFFT_TILED_BOTH(double, 96, 4, 1, 256, 8, 8, 16, 8)
+DFFT_TILED_BOTH(double, 96, 4, 0, 512, 16, 4, 16, 16)
+DFFT_TILED_BOTH(double, 96, 4, 1, 512, 16, 4, 16, 16)
+DFFT_TILED_BOTH(float, 160, 4, 0, 128, 8, 16, 8, 8)
+DFFT_TILED_BOTH(float, 160, 4, 1, 128, 8, 16, 8, 8)
+DFFT_TILED_BOTH(float, 96, 4, 0, 256, 8, 8, 16, 8)
+DFFT_TILED_BOTH(float, 160, 4, 1, 256, 8, 16, 16, 8)
+DFFT_TILED_BOTH(float, 96, 4, 0, 512, 16, 4, 16, 16)
+DFFT_TILED_BOTH(float, 160, 4, 1, 512, 16, 8, 16, 16)
 
 #define E(DBL, T, LB, MINB, S, L, P, NST, RAD, C, ...)                                             \
   {DBL, L, P, NST, RAD, LB, C, S, 5, K(T, LB, MINB, S, 5, L, P, C, __VA_ARGS__)},                 \
       {DBL, L, P, NST, RAD, LB, C, S, 4, K(T, LB, MINB, S, 4, L, P, C, __VA_ARGS__)}
 #define R2(a, b) {a, b}
-#define R3(a, b, c) {a, b, c}
 
 static const TiledKernel kTiledKernels[] = {
-    // dbl, L, P, nst, radices, threads, C, strided, kind, kernel
-    E(1, double, 160, 3, 0, 128, 8, 2, R2(16, 8), 16, 16, 8),
-    E(1, double, 160, 3, 1, 128, 8, 2, R2(16, 8), 16, 16, 8),
-    E(1, double, 160, 3, 0, 256, 16, 2, R2(16, 16), 8, 16, 16),
-    E(1, double, 160, 3, 1, 256, 16, 2, R2(16, 16), 8, 16, 16),
-    E(1, double, 160, 3, 0, 512, 64, 3, R3(8, 8, 8), 2, 8, 8, 8),
-    E(1, double, 288, 2, 1, 512, 64, 3, R3(8, 8, 8), 4, 8, 8, 8),
-    E(0, float, 160, 3, 0, 128, 8, 2, R2(16, 8), 16, 16, 8),
-    E(0, float, 160, 3, 1, 128, 8, 2, R2(16, 8), 16, 16, 8),
-    E(0, float, 160, 3, 0, 256, 16, 2, R2(16, 16), 8, 16, 16),
-    E(0, float, 288, 2, 1, 256, 16, 2, R2(16, 16), 16, 16, 16),
-    E(0, float, 160, 3, 0, 512, 64, 3, R3(8, 8, 8), 2, 8, 8, 8),
-    E(0, float, 288, 2, 1, 512, 64, 3, R3(8, 8, 8), 4, 8, 8, 8),
+    // dbl, N, P, nst, radices of N/2, threads, C, strided, kind, kernel
+    E(1, double, 96, 4, 0, 128, 8, 2, R2(8, 8), 8, 8, 8),
+    E(1, double, 96, 4, 1, 128, 8, 2, R2(8, 8), 8, 8, 8),
+    E(1, double, 96, 4, 0, 256, 8, 2, R2(16, 8), 8, 16, 8),
+    E(1, double, 96, 4, 1, 256, 8, 2, R2(16, 8), 8, 16, 8),
+    E(1, double, 96, 4, 0, 512, 16, 2, R2(16, 16), 4, 16, 16),
+    E(1, double, 96, 4, 1, 512, 16, 2, R2(16, 16), 4, 16, 16),
+    E(0, float, 160, 4, 0, 128, 8, 2, R2(8, 8), 16, 8, 8),
+    E(0, float, 160, 4, 1, 128, 8, 2, R2(8, 8), 16, 8, 8),
+    E(0, float, 96, 4, 0, 256, 8, 2, R2(16, 8), 8, 16, 8),
+    E(0, float, 160, 4, 1, 256, 8, 2, R2(16, 8), 16, 16, 8),
+    E(0, float, 96, 4, 0, 512, 16, 2, R2(16, 16), 4, 16, 16),
+    E(0, float, 160, 4, 1, 512, 16, 2, R2(16, 16), 8, 16, 16),
 };
 
 #undef E

@@ -1,43 +1,64 @@
 // Tile-staged R2R passes for DCT-II / DCT-III (FFTW REDFT10 / REDFT01, the
 // R2R(...) kinds of src/fft.jl:1-11 the README's 2-D DCT uses): a producer
 // warp moves whole input tiles into NB shared-memory buffers -- C whole
-// pencils by one 1-D bulk copy along the contiguous axis (STRIDED = 0), C
-// columns x n rows by TMA boxes of the real tensor {I, n, O} along a strided
-// axis (STRIDED = 1) -- and the stage threads run the stages with the kind's
-// load map (first stage) and store map (last stage) applied while reading
-// and writing the tile, compiled in for the kind (r2r_load / r2r_store);
-// every read of a tile precedes the first stage's barrier, so the output
-// overwrites the input in place, and the tile leaves by the same kind of
-// copy, which the producer issues when the buffer is handed back.  The FFT runs in a padded complex work buffer, one column per C.
-// Bounded waits as in the other pipelined passes.
+// pencils, one 1-D bulk copy each, along the contiguous axis (STRIDED = 0), C
+// columns x N rows by TMA boxes of the real tensor {I, N, O} along a strided
+// axis (STRIDED = 1) -- and the output leaves from the same buffer by the
+// same kind of copy, which the producer issues when the buffer is handed back.
+//
+// Both kinds are a permutation of N reals around a real transform, which runs
+// as one complex FFT of M = N/2 points (x the input, v its permutation, w =
+// exp(-2 pi i / N), c_j = exp(-i pi j / 2N)):
+//   DCT-II: v_k = x_{2k} | x_{2N-2k-1}; z_m = v_{2m} + i v_{2m+1}; Z = FFT_M(z);
+//     E = (Z_k + conj Z_{M-k})/2, T = -i w^k (Z_k - conj Z_{M-k})/2,
+//     V_k = E + T, V_{M-k} = conj(E - T); with q = c_j V_j:
+//     Y_j = 2 Re q, Y_{N-j} = -2 Im q.
+//   DCT-III: V_j = conj(c_j) (x_j - i x_{N-j}), x_N = 0; A = V_k, B = conj
+//     V_{M-k}, S = A + B, U = i conj(w^k) (A - B), Z_k = S + U, Z_{M-k} =
+//     conj(S - U); z = IFFT_M(Z) (unnormalised); v_{2m} = Re z_m, v_{2m+1} =
+//     Im z_m, stored at the permuted places.
+// (A complex FFT of the N reals with zero imaginary parts took twice the
+// FP64 work and shared-memory traffic: 256 x 256 x 32 Float64 DCT-II +
+// DCT-III, four passes, 54 us.)  The FFT runs in a padded complex work
+// buffer, one column per real column; columns stay independent of one
+// another.  Bounded waits as in the other pipelined passes.
 #pragma once
 #include "real_pass.cuh"
 
 namespace dfft {
 
-// The tile of one column / pencil seen through a kind's maps (stride S
+// Place of v_k in the data: x_{2k} | x_{2N-2k-1}.
+template <int N> __device__ __forceinline__ int dct_place(int k) { return 2 * k < N ? 2 * k : 2 * N - 2 * k - 1; }
+// The tile of one column / pencil as the packed sequence z_m (stride S
 // between its elements: C in a strided tile, 1 in a contiguous one).
-template <typename T, int KIND, int S> struct R2RLoadView {
-  typedef typename cvec<T>::type V;
-  const T* p;
-  int N;
-  const V* w;
-  __device__ __forceinline__ V ld(int b, int off) const { return r2r_load<T, KIND>(p, 0, S, N, w, b + off); }
-};
-template <typename T, int KIND, int S> struct R2RStoreView {
+template <typename T, int N, int S> struct DctView {
   typedef typename cvec<T>::type V;
   T* p;
-  int N;
-  const V* w;
+  __device__ __forceinline__ V ld(int b, int off) const {
+    const int m = b + off;
+    return mk<V>(p[dct_place<N>(2 * m) * S], p[dct_place<N>(2 * m + 1) * S]);
+  }
   __device__ __forceinline__ void st(int b, int off, V v) const {
-    r2r_store<T, KIND>(p, 0, S, N, w, b + off, v, (T)1);
+    const int m = b + off;
+    p[dct_place<N>(2 * m) * S] = v.x;
+    p[dct_place<N>(2 * m + 1) * S] = v.y;
   }
 };
+
+// Barrier of the BAR stage threads after a loop whose last round is not every
+// lane's: the form that does not need a converged warp.  (With bar.sync, as
+// in stage_sync, a warp that reaches the barrier in two halves hangs; the
+// compiler may send the lanes of the last round, tid < 16 in a strided tile,
+// past it on a copy of their own, since only they can meet the tid == 0 test
+// that follows.)
+template <int BAR> __device__ __forceinline__ void loop_sync() {
+  __syncwarp();
+  asm volatile("barrier.cta.sync 1, %0;" ::"n"(BAR) : "memory");
+}
 
 struct TiledGeom {
   long long ntiles;  // contiguous: pencils / C; strided: tiles_i * O
   int tiles_i;       // strided: tiles along I
-  int n_in, n_out;   // elements per pencil / rows per column (side type T)
   int lb, nlb;       // strided: rows per TMA box, boxes per tile
   int ld;            // padded complex work elements per column
   int bstride;       // bytes between tile buffers (128-byte multiple)
@@ -46,12 +67,15 @@ struct TiledGeom {
   int* err;
 };
 
-template <typename T, int LB, int MINB, int NB, int STRIDED, int KIND, int L, int P, int C, int... Rs>
+template <typename T, int LB, int MINB, int NB, int STRIDED, int KIND, int N, int P, int C, int... Rs>
 __global__ void __launch_bounds__(LB, MINB)
     tiled_pass(const PassDesc d, const __grid_constant__ CUtensorMap tin,
                const __grid_constant__ CUtensorMap tout, const TiledGeom g) {
   typedef typename cvec<T>::type V;
   constexpr int NC = C * P;
+  constexpr int M = N / 2;                     // FFT length
+  constexpr int ROUNDS = M / 2 / P + 1;        // of the split / merge loops over k <= M/2
+  constexpr int PS = N + 64 / (int)sizeof(T);  // contiguous tiles: elements between pencils (spread over the banks)
   static_assert(NC % 32 == 0 && NC + 32 == LB, "whole warps of stage threads plus one producer warp");
   static_assert(NB >= 2 && NB <= 4, "tile buffers");
   extern __shared__ __align__(128) unsigned char smem_tiled[];
@@ -84,8 +108,7 @@ __global__ void __launch_bounds__(LB, MINB)
   if (tid >= NC) {
     if (tid == NC) {
       // ---------------- producer ----------------
-      const uint32_t in_bytes = (uint32_t)((size_t)C * g.n_in * sizeof(T));
-      const uint32_t out_bytes = (uint32_t)((size_t)C * g.n_out * sizeof(T));
+      const uint32_t tile_bytes = (uint32_t)((size_t)C * N * sizeof(T));
       int fills[NB] = {};
       long long pend[NB];  // transformed tile in buffer b still to be stored, or -1
       for (int bb = 0; bb < NB; ++bb) pend[bb] = -1;
@@ -102,7 +125,9 @@ __global__ void __launch_bounds__(LB, MINB)
           for (int kb = 0; kb < g.nlb; ++kb)
             tma_store_3d(&tout, buf + (size_t)kb * g.lb * C * sizeof(T), ti * C, kb * g.lb, o);
         } else {
-          bulk_store_1d(reinterpret_cast<T*>(g.dst) + pend[b] * C * g.n_out, buf, out_bytes);
+          for (int cc = 0; cc < C; ++cc)
+            bulk_store_1d(reinterpret_cast<T*>(g.dst) + (pend[b] * C + cc) * N, buf + (size_t)cc * PS * sizeof(T),
+                          (uint32_t)(N * sizeof(T)));
         }
         bulk_commit();
         bulk_wait_read_all();
@@ -124,14 +149,16 @@ __global__ void __launch_bounds__(LB, MINB)
           break;
         }
         unsigned char* buf = bufs + b * bst;
-        mbar_expect_tx(&full[b], in_bytes);
+        mbar_expect_tx(&full[b], tile_bytes);
         if (STRIDED) {
           const int ti = (int)(tile % g.tiles_i);
           const int o = (int)(tile / g.tiles_i);
           for (int kb = 0; kb < g.nlb; ++kb)
             tma_load_3d(buf + (size_t)kb * g.lb * C * sizeof(T), &tin, &full[b], ti * C, kb * g.lb, o);
         } else {
-          bulk_load_1d(buf, reinterpret_cast<const T*>(g.src) + tile * C * g.n_in, in_bytes, &full[b]);
+          for (int cc = 0; cc < C; ++cc)
+            bulk_load_1d(buf + (size_t)cc * PS * sizeof(T), reinterpret_cast<const T*>(g.src) + (tile * C + cc) * N,
+                         (uint32_t)(N * sizeof(T)), &full[b]);
         }
         pend[b] = tile;
         tile += gridDim.x;
@@ -151,14 +178,8 @@ __global__ void __launch_bounds__(LB, MINB)
     const GlobalTw<V> tw{reinterpret_cast<const V*>(d.tw)};
     constexpr int S = STRIDED ? C : 1;
     constexpr int DIR = KIND == K_REDFT01 ? 2 : 1;  // REDFT01 runs as an inverse FFT
-    typedef R2RLoadView<T, KIND, S> In;
-    typedef R2RStoreView<T, KIND, S> Out;
-    // the tile's element (column c, row / element k) sits at c + k*C
-    // (strided) or c*n + k (contiguous)
-    const size_t ib = STRIDED ? c : (size_t)c * g.n_in;
-    const size_t ob = STRIDED ? c : (size_t)c * g.n_out;
-    const V* w_in = reinterpret_cast<const V*>(d.in.w);
-    const V* w_out = reinterpret_cast<const V*>(d.out.w);
+    const V* w = reinterpret_cast<const V*>(d.tw2);  // w^k, k <= M/2
+    const V* cj = reinterpret_cast<const V*>(KIND == K_REDFT01 ? d.in.w : d.out.w);  // conj(c_j) / c_j
     for (int it = 0;; ++it) {
       const int b = it % NB;
       if (!mbar_wait_bounded(&full[b], (uint32_t)((it / NB) & 1))) s_cabort = 1;
@@ -167,12 +188,44 @@ __global__ void __launch_bounds__(LB, MINB)
       const long long tile = s_tile[b];
       if (tile < 0) break;
       unsigned char* buf = bufs + b * bst;
-      const In in{reinterpret_cast<const T*>(buf) + ib, d.in.n, w_in};
-      const Out out{reinterpret_cast<T*>(buf) + ob, d.out.n, w_out};
-      static_stages<T, L, P, 1, NC, DIR, 1, 1, 0, In, PadCol<V>, Out, GlobalTw<V>, Rs...>(d, t, in, col, out,
-                                                                                            tw, 0, 0, true);
+      T* x = reinterpret_cast<T*>(buf) + (STRIDED ? c : c * PS);  // element n at x[n * S]
+      const DctView<T, N, S> view{x};
+      if constexpr (KIND == K_REDFT01) {
+#pragma unroll 1
+        for (int i = 0; i < ROUNDS; ++i) {
+          const int k = t + i * P;
+          if (k > M / 2) continue;
+          const T xn = k == 0 ? (T)0 : x[(N - k) * S];
+          const V A = cmul(ldg_c(cj + k), mk<V>(x[k * S], -xn));
+          const V B = cconj(cmul(ldg_c(cj + M - k), mk<V>(x[(M - k) * S], -x[(M + k) * S])));
+          const V U = cmul_pi(cmul(cconj(ldg_c(w + k)), csub(A, B)));
+          const V Z = cadd(A, B);
+          col.st(k, 0, cadd(Z, U));
+          if (k > 0) col.st(M - k, 0, cconj(csub(Z, U)));
+        }
+        loop_sync<NC>();
+        static_stages<T, M, P, 1, NC, DIR, 1, 1, 0, PadCol<V>, PadCol<V>, DctView<T, N, S>, GlobalTw<V>, Rs...>(
+            d, t, col, col, view, tw, 0, 0, true);
+      } else {
+        static_stages<T, M, P, 1, NC, DIR, 1, 1, 0, DctView<T, N, S>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(
+            d, t, view, col, col, tw, 0, 0, true);
+#pragma unroll 1
+        for (int i = 0; i < ROUNDS; ++i) {
+          const int k = t + i * P;
+          if (k > M / 2) continue;
+          const V zk = col.ld(k, 0), zm = cconj(col.ld(k == 0 ? 0 : M - k, 0));
+          const V E = cscale(cadd(zk, zm), (T)0.5);
+          const V U = cmul(ldg_c(w + k), cscale(cmul_mi(csub(zk, zm)), (T)0.5));
+          const V q = cmul(ldg_c(cj + k), cadd(E, U));
+          const V r = cmul(ldg_c(cj + M - k), cconj(csub(E, U)));
+          x[k * S] = (T)2 * q.x;
+          if (k > 0) x[(N - k) * S] = (T)-2 * q.y;
+          x[(M - k) * S] = (T)2 * r.x;
+          x[(M + k) * S] = k == 0 ? (T)2 * r.x : (T)-2 * r.y;
+        }
+      }
       fence_proxy_async_smem();  // the producer's store reads the tile next
-      stage_sync<NC>();
+      loop_sync<NC>();
       if (tid == 0) mbar_arrive(&empty[b]);  // hand the transformed tile to the producer
     }
     if (tid == 0 && s_cabort && *verr == 0) atomicExch(g.err, DFFT_DEVERR_TMA_TIMEOUT);
