@@ -119,7 +119,8 @@ struct TiledKernel {
   int kind;     // FFTW r2r kind (REDFT10 / REDFT01)
   const void* fn;
 };
-const TiledKernel* find_tiled_kernel(int dbl, int L, int strided, int kind);
+// The first with tiles of at most `most` columns, or null.
+const TiledKernel* find_tiled_kernel(int dbl, int L, int strided, int kind, long long most);
 // A compiled one-launch Bluestein pass (chirp_pass.cu): convolution length
 // M = r0 * r1, strided and contiguous kernels.
 struct ChirpKernel {

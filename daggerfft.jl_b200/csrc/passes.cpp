@@ -575,7 +575,9 @@ static Pass make_tiled_pass(const PassSpec& s) {
   const int kind = tiled_kind(s);
   const int L = s.L / 2;  // FFT of the N reals packed in pairs
   const int rsz = s.dbl ? 8 : 4, csz = 2 * rsz;
-  const TiledKernel* k = kind ? find_tiled_kernel(s.dbl, s.L, kind == 2 ? 1 : 0, s.in.r2r) : nullptr;
+  const TiledKernel* k = kind ? find_tiled_kernel(s.dbl, s.L, kind == 2 ? 1 : 0, s.in.r2r,
+                                                   kind == 2 ? s.I : 1LL << 30)
+                               : nullptr;
   if (!k) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "no tiled kernel for this pass"};
   const int n = s.in.n;
   const int C = k->cs;
@@ -587,9 +589,10 @@ static Pass make_tiled_pass(const PassSpec& s) {
   p.fn = k->fn;
   TiledGeom& g = p.tgeom;
   if (kind == 1) {
-    if (s.O % C != 0 || ((size_t)C * n * rsz) % 16 != 0)
-      throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "pencils do not split into whole tiles"};
-    g.ntiles = s.O / C;
+    if (((size_t)n * rsz) % 16 != 0)
+      throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "pencils are not bulk copies"};
+    g.pencils = s.O;
+    g.ntiles = (s.O + C - 1) / C;
     g.tiles_i = 1;
     g.lb = n;
     g.nlb = 1;

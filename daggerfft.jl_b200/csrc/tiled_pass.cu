@@ -29,6 +29,7 @@ DFFT_TILED_BOTH(float, 96, 4, 0, 256, 8, 8, 16, 8)
 DFFT_TILED_BOTH(float, 160, 4, 1, 256, 8, 16, 16, 8)
 DFFT_TILED_BOTH(float, 96, 4, 0, 512, 16, 4, 16, 16)
 DFFT_TILED_BOTH(float, 160, 4, 1, 512, 16, 8, 16, 16)
+DFFT_TILED_BOTH(float, 96, 4, 1, 512, 16, 4, 16, 16)
 
 #define E(DBL, T, LB, MINB, S, L, P, NST, RAD, C, ...)                                             \
   {DBL, L, P, NST, RAD, LB, C, S, 5, K(T, LB, MINB, S, 5, L, P, C, __VA_ARGS__)},                 \
@@ -49,14 +50,15 @@ static const TiledKernel kTiledKernels[] = {
     E(0, float, 160, 4, 1, 256, 8, 2, R2(16, 8), 16, 16, 8),
     E(0, float, 96, 4, 0, 512, 16, 2, R2(16, 16), 4, 16, 16),
     E(0, float, 160, 4, 1, 512, 16, 2, R2(16, 16), 8, 16, 16),
+    E(0, float, 96, 4, 1, 512, 16, 2, R2(16, 16), 4, 16, 16),  // arrays of 4 columns
 };
 
 #undef E
 #undef K
 
-const TiledKernel* find_tiled_kernel(int dbl, int L, int strided, int kind) {
+const TiledKernel* find_tiled_kernel(int dbl, int L, int strided, int kind, long long most) {
   for (const TiledKernel& k : kTiledKernels)
-    if (k.dbl == dbl && k.L == L && k.strided == strided && k.kind == kind) return &k;
+    if (k.dbl == dbl && k.L == L && k.strided == strided && k.kind == kind && k.cs <= most) return &k;
   return nullptr;
 }
 

@@ -57,7 +57,8 @@ template <int BAR> __device__ __forceinline__ void loop_sync() {
 }
 
 struct TiledGeom {
-  long long ntiles;  // contiguous: pencils / C; strided: tiles_i * O
+  long long ntiles;  // contiguous: ceil(pencils / C); strided: tiles_i * O
+  long long pencils; // contiguous: pencils in all (the last tile may hold fewer than C)
   int tiles_i;       // strided: tiles along I
   int lb, nlb;       // strided: rows per TMA box, boxes per tile
   int ld;            // padded complex work elements per column
@@ -108,7 +109,6 @@ __global__ void __launch_bounds__(LB, MINB)
   if (tid >= NC) {
     if (tid == NC) {
       // ---------------- producer ----------------
-      const uint32_t tile_bytes = (uint32_t)((size_t)C * N * sizeof(T));
       int fills[NB] = {};
       long long pend[NB];  // transformed tile in buffer b still to be stored, or -1
       for (int bb = 0; bb < NB; ++bb) pend[bb] = -1;
@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(LB, MINB)
           for (int kb = 0; kb < g.nlb; ++kb)
             tma_store_3d(&tout, buf + (size_t)kb * g.lb * C * sizeof(T), ti * C, kb * g.lb, o);
         } else {
-          for (int cc = 0; cc < C; ++cc)
+          const int nv = (int)min((long long)C, g.pencils - pend[b] * C);
+          for (int cc = 0; cc < nv; ++cc)
             bulk_store_1d(reinterpret_cast<T*>(g.dst) + (pend[b] * C + cc) * N, buf + (size_t)cc * PS * sizeof(T),
                           (uint32_t)(N * sizeof(T)));
         }
@@ -149,14 +150,15 @@ __global__ void __launch_bounds__(LB, MINB)
           break;
         }
         unsigned char* buf = bufs + b * bst;
-        mbar_expect_tx(&full[b], tile_bytes);
+        const int nv = STRIDED ? C : (int)min((long long)C, g.pencils - tile * C);
+        mbar_expect_tx(&full[b], (uint32_t)((size_t)nv * N * sizeof(T)));
         if (STRIDED) {
           const int ti = (int)(tile % g.tiles_i);
           const int o = (int)(tile / g.tiles_i);
           for (int kb = 0; kb < g.nlb; ++kb)
             tma_load_3d(buf + (size_t)kb * g.lb * C * sizeof(T), &tin, &full[b], ti * C, kb * g.lb, o);
         } else {
-          for (int cc = 0; cc < C; ++cc)
+          for (int cc = 0; cc < nv; ++cc)
             bulk_load_1d(buf + (size_t)cc * PS * sizeof(T), reinterpret_cast<const T*>(g.src) + (tile * C + cc) * N,
                          (uint32_t)(N * sizeof(T)), &full[b]);
         }

@@ -47,3 +47,26 @@ def test_dct_stack_uses_tiles(order):
     assert rel(to_np(F), ref) <= 1e-12
     B = dfft.fft(F, dims=(1, 2), transforms=(dfft.R2R((dfft.REDFT01, dfft.REDFT01)),))
     assert rel(to_np(B), a * (2 * 256) ** 2) <= 1e-12
+
+
+@pytest.mark.parametrize("n", [128, 256, 512])
+@pytest.mark.parametrize("cols", [1, 4, 13])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", [dfft.REDFT10, dfft.REDFT01])
+def test_column_counts_that_do_not_fill_a_tile(n, cols, dtype, kind):
+    # contiguous pencils whose last tile is partial, and few strided columns;
+    # an infinity stays in its own column
+    a = rand((n, cols), dtype, seed=n + cols)
+    tr = (dfft.R2R((kind,)),)
+    p = dfft.gpu_plan_transform(dfft.R2R((kind,)), to_gpu(a), (1,))
+    assert p.describe().startswith("tiled-contig"), p.describe()
+    ref = oracle.fft(a, dims=(1,), transforms=(oracle.R2R((kind,)),))
+    assert rel(to_np(dfft.fft(to_gpu(a), dims=(1,), transforms=tr)), ref) <= tol_for(dtype)
+    b = np.ascontiguousarray(a.T)
+    y = to_np(dfft.fft(to_gpu(b), dims=(2,), transforms=tr))
+    assert rel(y, np.asarray(ref).T) <= tol_for(dtype)
+    if cols > 1:
+        a[3, cols - 1] = np.inf
+        y = to_np(dfft.fft(to_gpu(a), dims=(1,), transforms=tr))
+        assert np.isfinite(y[:, :-1]).all() and not np.isfinite(y[:, -1]).all()
+        assert rel(y[:, :-1], np.asarray(ref)[:, :-1]) <= tol_for(dtype)
