@@ -282,7 +282,23 @@ template <typename V> struct StageTwG {
 // Barrier between the stages: the whole CTA (BAR = 0) or named barrier 1
 // over the BAR threads that run the stages (the other warps of the CTA do
 // something else, e.g. feed the tile pipeline).
+// The lanes of a warp may come to it apart: after a wait each lane polls for
+// itself, a loop whose last round is not every lane's, stores behind a
+// condition.  (bar.sync is the aligned form: a warp that reaches it in two
+// parts hangs, and the compiler may well send the lanes of a loop's last
+// round past it on a copy of their own, for instance where only they can meet
+// the tid == 0 test that follows.)
 template <int BAR> __device__ __forceinline__ void stage_sync() {
+  if constexpr (BAR == 0) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(BAR) : "memory");
+  }
+}
+// The aligned form, for code without a branch since the last stage_sync: the
+// stages in which every thread has the same number of butterflies.
+template <int BAR> __device__ __forceinline__ void stage_sync_converged() {
   if constexpr (BAR == 0) __syncthreads();
   else asm volatile("bar.sync 1, %0;" ::"n"(BAR) : "memory");
 }
@@ -342,7 +358,10 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
       }
     }
   }
-  if (!from_global) stage_sync<BAR>();
+  if (!from_global) {
+    if (exact) stage_sync_converged<BAR>();
+    else stage_sync<BAR>();
+  }
 #pragma unroll
   for (int b = 0; b < BMAX; ++b) {
     const int j = CLAMP && !exact ? min(t + b * P, Lr - 1) : t + b * P;
@@ -377,7 +396,10 @@ __device__ __forceinline__ void stage_body(const PassDesc& d, int L, int P, int 
       }
     }
   }
-  if (!to_global) stage_sync<BAR>();
+  if (!to_global) {
+    if (exact) stage_sync_converged<BAR>();
+    else stage_sync<BAR>();
+  }
 }
 
 // Shared prologue: thread -> (column, butterfly lane), column base offsets.

@@ -164,8 +164,11 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
         static_stages<T, M, P, 1, NC, 1, 1, 1, 0, StrideCol<V>, PadCol<V>, PadCol<V>, StageTw<V>, Rs...>(
             d, t, padded, pad, pad, tw, 0, 0, true);
         // post-pass: X_k of pencil cc, k = 0..M, into the consumed tile
-        // buffer, dense: element e = cc*(M+1) + k
-        for (int e = tid; e < C * (M + 1); e += NC) {
+        // buffer, dense: element e = cc*(M+1) + k (the last round is some
+        // threads' only: 16 of 96 at M = 48)
+        for (int i = 0; i < (C * (M + 1) + NC - 1) / NC; ++i) {
+          const int e = tid + i * NC;
+          if (e >= C * (M + 1)) continue;
           const int cc = e / (M + 1), k = e - cc * (M + 1);
           const PadCol<V> z{work + (size_t)cc * g.ld};
           const V zk = z.ld(k == M ? 0 : k, 0);
@@ -177,7 +180,9 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
       } else {
         // pre-pass: Z'_k of pencil cc, k = 0..M-1, from the dense tile
         // (element cc*(M+1) + k) into the work buffer
-        for (int e = tid; e < C * M; e += NC) {
+        for (int i = 0; i < (C * M + NC - 1) / NC; ++i) {
+          const int e = tid + i * NC;
+          if (e >= C * M) continue;
           const int cc = e / M, k = e - cc * M;
           const V* x = buf + (size_t)cc * (M + 1);
           V A = x[k];
@@ -189,13 +194,15 @@ __global__ void __launch_bounds__(LB, MINB) real_pass(const PassDesc d, const Re
           const PadCol<V> z{work + (size_t)cc * g.ld};
           z.st(k, 0, cadd(cadd(A, B), cmul_pi(cmul(cconj(sw[k]), csub(A, B)))));
         }
-        stage_sync<NC>();
+        if constexpr (C * M % NC == 0) stage_sync_converged<NC>();
+        else stage_sync<NC>();
         const StrideCol<V> padded{buf + (size_t)c * PS, 1};
         static_stages<T, M, P, 1, NC, 2, 1, 1, 0, PadCol<V>, PadCol<V>, StrideCol<V>, StageTw<V>, Rs...>(
             d, t, pad, pad, padded, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the producer's bulk store reads the tile next
-      stage_sync<NC>();
+      if constexpr (DIR == 2) stage_sync_converged<NC>();  // the stages end in a barrier
+      else stage_sync<NC>();
       if (tid == 0) mbar_arrive(&empty[b]);  // hand the transformed tile to the producer
     }
     if (tid == 0 && s_cabort && *verr == 0) atomicExch(g.err, DFFT_DEVERR_TMA_TIMEOUT);

@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(LB, MINB)
                       TWT, Rs...>(dy, t, dense, sw, dense, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the buffer is next read (store) or written (load) by TMA
-      stage_sync<NC>();
+      stage_sync_converged<NC>();
       if (tid == 0) mbar_arrive(&empty[b]);  // the producer publishes (x) or stores (y) the tile
     }
     if (tid == 0 && s_cabort && *verr == 0) atomicExch(g.err, DFFT_DEVERR_TMA_TIMEOUT);
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(LB, MINB)
                       StrideColC<V, CS>, StageTw<V>, Rs...>(d, t, dense, dense, dense, tw, 0, 0, true);
       }
       fence_proxy_async_smem();  // the producer's TMA store reads the tile next
-      stage_sync<NC>();
+      stage_sync_converged<NC>();
       if (tid == 0) mbar_arrive(&empty[b]);  // hand the transformed tile to the producer
     }
     if (tid == 0 && s_cabort && *verr == 0) atomicExch(g.err, DFFT_DEVERR_TMA_TIMEOUT);

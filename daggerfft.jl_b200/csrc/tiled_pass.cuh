@@ -45,17 +45,6 @@ template <typename T, int N, int S> struct DctView {
   }
 };
 
-// Barrier of the BAR stage threads after a loop whose last round is not every
-// lane's: the form that does not need a converged warp.  (With bar.sync, as
-// in stage_sync, a warp that reaches the barrier in two halves hangs; the
-// compiler may send the lanes of the last round, tid < 16 in a strided tile,
-// past it on a copy of their own, since only they can meet the tid == 0 test
-// that follows.)
-template <int BAR> __device__ __forceinline__ void loop_sync() {
-  __syncwarp();
-  asm volatile("barrier.cta.sync 1, %0;" ::"n"(BAR) : "memory");
-}
-
 struct TiledGeom {
   long long ntiles;  // contiguous: ceil(pencils / C); strided: tiles_i * O
   long long pencils; // contiguous: pencils in all (the last tile may hold fewer than C)
@@ -205,7 +194,7 @@ __global__ void __launch_bounds__(LB, MINB)
           col.st(k, 0, cadd(Z, U));
           if (k > 0) col.st(M - k, 0, cconj(csub(Z, U)));
         }
-        loop_sync<NC>();
+        stage_sync<NC>();
         static_stages<T, M, P, 1, NC, DIR, 1, 1, 0, PadCol<V>, PadCol<V>, DctView<T, N, S>, GlobalTw<V>, Rs...>(
             d, t, col, col, view, tw, 0, 0, true);
       } else {
@@ -227,7 +216,7 @@ __global__ void __launch_bounds__(LB, MINB)
         }
       }
       fence_proxy_async_smem();  // the producer's store reads the tile next
-      loop_sync<NC>();
+      stage_sync<NC>();
       if (tid == 0) mbar_arrive(&empty[b]);  // hand the transformed tile to the producer
     }
     if (tid == 0 && s_cabort && *verr == 0) atomicExch(g.err, DFFT_DEVERR_TMA_TIMEOUT);

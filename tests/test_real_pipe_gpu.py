@@ -59,3 +59,33 @@ def test_known_answers():
     assert np.abs(F - e).max() <= 1e-11
     x = to_np(dfft.irfft(to_gpu(e), n, dims=(1,)))
     assert np.abs(x - a).max() <= 1e-14
+
+
+@pytest.mark.parametrize("m", HALF)
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_several_tiles_per_cta(m, dtype):
+    # the split and pack loops end in a round of only some lanes (16 of 96
+    # threads at m = 48): the barrier after it in every tile of a CTA
+    n, o = 2 * m, 32 * 1999
+    a = rand((n, o), dtype, seed=m + 1)
+    F = dfft.rfft(to_gpu(a), dims=(1,))
+    ref = np.fft.rfft(a.astype(np.float64), axis=0)
+    assert rel(to_np(F), ref) <= tol_for(dtype)
+    x = dfft.irfft(F, n, dims=(1,))
+    assert rel(to_np(x), a) <= tol_for(dtype)
+    assert dfft.device_error() == 0
+
+
+@pytest.mark.parametrize("L", [192, 384])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_uneven_butterflies_in_the_slab_pass(L, dtype):
+    # 12 x 16 and 24 x 16 over 16 threads: stages whose stores are some lanes' only
+    a = rand((L, L, 6), dtype, seed=L)
+    g = to_gpu(a)
+    p = dfft.gpu_plan_transform(dfft.FFT(), g, (1, 2), flags=dfft.FLAG_FUSE)
+    assert p.describe().startswith("slab-xy"), p.describe()
+    out = dfft.empty_like_layout(p.out_shape, g.dtype, g)
+    for _ in range(4):
+        p.execute(g, out)
+    assert rel(to_np(out), np.fft.fft2(a.astype(np.complex128), axes=(0, 1))) <= tol_for(dtype)
+    assert dfft.device_error() == 0
