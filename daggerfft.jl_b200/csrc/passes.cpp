@@ -168,6 +168,25 @@ void load_encode() {
       q == cudaDriverEntryPointSuccess)
     g_encode = reinterpret_cast<EncodeTiledFn>(fn);
 }
+
+// cuTensorMapEncodeTiled for a 3-D tensor of unswizzled or swizzled boxes.  A
+// driver call: it needs the device's context bound to the thread, which a
+// thread that has made no runtime call beyond cudaGetDevice does not have yet
+// (cudaSetDevice binds it).
+cudaError_t encode_3d(CUtensorMap* m, CUtensorMapDataType type, void* base, const cuuint64_t* dims,
+                      const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+  std::call_once(g_encode_once, load_encode);
+  if (!g_encode) return cudaErrorNotSupported;
+  const cuuint32_t estr[3] = {1, 1, 1};
+  for (int attempt = 0;; ++attempt) {
+    const CUresult r = g_encode(m, type, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) return cudaSuccess;
+    int dev = 0;
+    if (attempt || cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess)
+      return cudaErrorInvalidValue;
+  }
+}
 }  // namespace
 
 int* device_error_word() {
@@ -185,33 +204,22 @@ int* device_error_word() {
 
 // Tensor map over the real tensor {I, n, O} of a strided tiled pass.
 static cudaError_t encode_real_map(CUtensorMap* m, void* base, const Pass& p, int dbl) {
-  std::call_once(g_encode_once, load_encode);
-  if (!g_encode) return cudaErrorNotSupported;
   const cuuint64_t esz = dbl ? 8 : 4;
-  cuuint64_t dims[3] = {(cuuint64_t)p.tI, (cuuint64_t)p.tL, (cuuint64_t)p.tO};
-  cuuint64_t strides[2] = {(cuuint64_t)p.tI * esz, (cuuint64_t)p.tI * esz * (cuuint64_t)p.tL};
-  cuuint32_t box[3] = {(cuuint32_t)p.geom.C, (cuuint32_t)p.geom.lb, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(m, dbl ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  const cuuint64_t dims[3] = {(cuuint64_t)p.tI, (cuuint64_t)p.tL, (cuuint64_t)p.tO};
+  const cuuint64_t strides[2] = {(cuuint64_t)p.tI * esz, (cuuint64_t)p.tI * esz * (cuuint64_t)p.tL};
+  const cuuint32_t box[3] = {(cuuint32_t)p.geom.C, (cuuint32_t)p.geom.lb, 1};
+  return encode_3d(m, dbl ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides,
+                   box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 static cudaError_t encode_map_dims(CUtensorMap* m, void* base, const Pass& p, long long tI, long long tL,
                                    long long tO) {
-  std::call_once(g_encode_once, load_encode);
-  if (!g_encode) return cudaErrorNotSupported;
   const cuuint64_t esz = 8;
   const cuuint64_t xs = (cuuint64_t)p.geom.xscale;
-  cuuint64_t dims[3] = {(cuuint64_t)tI * xs, (cuuint64_t)tL, (cuuint64_t)tO};
-  cuuint64_t strides[2] = {(cuuint64_t)tI * xs * esz, (cuuint64_t)tI * xs * esz * (cuuint64_t)tL};
-  cuuint32_t box[3] = {(cuuint32_t)(p.geom.C * p.geom.xscale), (cuuint32_t)p.geom.lb, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, base, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  const cuuint64_t dims[3] = {(cuuint64_t)tI * xs, (cuuint64_t)tL, (cuuint64_t)tO};
+  const cuuint64_t strides[2] = {(cuuint64_t)tI * xs * esz, (cuuint64_t)tI * xs * esz * (cuuint64_t)tL};
+  const cuuint32_t box[3] = {(cuuint32_t)(p.geom.C * p.geom.xscale), (cuuint32_t)p.geom.lb, 1};
+  return encode_3d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 static cudaError_t encode_map(CUtensorMap* m, void* base, const Pass& p) {
@@ -221,16 +229,10 @@ static cudaError_t encode_map(CUtensorMap* m, void* base, const Pass& p) {
 // Tensor map over {I, L, O} ComplexF32 (8-byte elements) with boxes of 16
 // columns x 256 rows in the 128-byte swizzle the mixed pass reads and writes.
 static cudaError_t encode_map_sw128(CUtensorMap* m, void* base, const Pass& p) {
-  std::call_once(g_encode_once, load_encode);
-  if (!g_encode) return cudaErrorNotSupported;
-  cuuint64_t dims[3] = {(cuuint64_t)p.tI, (cuuint64_t)p.tL, (cuuint64_t)p.tO};
-  cuuint64_t strides[2] = {(cuuint64_t)p.tI * 8, (cuuint64_t)p.tI * 8 * (cuuint64_t)p.tL};
-  cuuint32_t box[3] = {16, (cuuint32_t)p.mgeom.lb, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, base, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  const cuuint64_t dims[3] = {(cuuint64_t)p.tI, (cuuint64_t)p.tL, (cuuint64_t)p.tO};
+  const cuuint64_t strides[2] = {(cuuint64_t)p.tI * 8, (cuuint64_t)p.tI * 8 * (cuuint64_t)p.tL};
+  const cuuint32_t box[3] = {16, (cuuint32_t)p.mgeom.lb, 1};
+  return encode_3d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 static int sm_count() {
