@@ -69,7 +69,7 @@ int dfft_plan_workspace_bytes(dfft_plan plan, size_t* bytes) {
   return guarded([&] {
     dfft::Plan* p = impl(plan);
     if (!bytes) throw Error{DFFT_ERROR_INVALID_VALUE, "bytes is NULL"};
-    *bytes = p->work_bytes + p->chirp_bytes;
+    *bytes = p->workspace_bytes();
   });
 }
 
@@ -117,6 +117,17 @@ int dfft_plan_describe(dfft_plan plan, char* buf, size_t len) {
 int dfft_execute(dfft_plan plan, const void* in, void* out, void* stream) {
   return guarded([&] {
     dfft::execute_plan(impl(plan), in, out, reinterpret_cast<cudaStream_t>(stream));
+  });
+}
+
+int dfft_execute_workspace(dfft_plan plan, const void* in, void* out, void* stream, void* workspace) {
+  return guarded([&] {
+    const dfft::Plan* p = impl(plan);
+    if (p->workspace_bytes() && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255)))
+      throw Error{DFFT_ERROR_INVALID_VALUE, "workspace is NULL or not 256-byte aligned"};
+    char* w = static_cast<char*>(workspace);
+    dfft::execute_plan(p, in, out, reinterpret_cast<cudaStream_t>(stream), p->work_bytes ? w : nullptr,
+                       p->chirp_bytes ? w + p->chirp_offset() : nullptr);
   });
 }
 

@@ -23,6 +23,9 @@ struct Plan {
   void* chirp = nullptr;          // Bluestein scratch (Q*M complex per axis, max over axes)
   size_t chirp_bytes = 0;
   ~Plan();
+  // one workspace of both: work first, chirp at a 256-byte boundary
+  size_t chirp_offset() const { return chirp_bytes ? (work_bytes + 255) & ~(size_t)255 : work_bytes; }
+  size_t workspace_bytes() const { return chirp_offset() + chirp_bytes; }
   size_t in_bytes() const;
   size_t out_bytes() const;
 };
@@ -37,14 +40,10 @@ Plan* build_slab_split_plan(int precision, int inverse, int64_t L, int64_t nslab
                             int split_dim, unsigned flags);
 
 // work / chirp: workspaces supplied by the caller for this execution (null:
-// the plan's own); a plan built with kFlagCallerWorkspace owns none.
+// the plan's own); a plan built with DFFT_FLAG_CALLER_WORKSPACE owns none.
 // overlap: the launches may overlap the tails of the kernels before them.
 void execute_plan(const Plan* p, const void* in, void* out, cudaStream_t stream, void* work = nullptr,
                   void* chirp = nullptr, bool overlap = true);
-
-// Internal plan flag (above the public DFFT_FLAG_* bits): allocate no
-// workspace; every execution brings its own (the serving runtime's arena).
-constexpr unsigned kFlagCallerWorkspace = 1u << 30;
 
 }  // namespace dfft
 

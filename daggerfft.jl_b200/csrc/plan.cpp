@@ -313,7 +313,7 @@ Plan* build_plan(int ndim, const int64_t* shape, int precision, int transform, i
     }
   }
   P->chirp_bytes = chirp_bytes;
-  if (!(flags & kFlagCallerWorkspace)) {
+  if (!(flags & DFFT_FLAG_CALLER_WORKSPACE)) {
     if (chirp_bytes) cuda_check(cudaMalloc(&P->chirp, chirp_bytes), "cudaMalloc(bluestein scratch)");
     if (P->work_bytes) cuda_check(cudaMalloc(&P->work, P->work_bytes), "cudaMalloc(workspace)");
   }
@@ -365,7 +365,7 @@ Plan* build_slab_split_plan(int precision, int inverse, int64_t L, int64_t nslab
     }
   }
   if (!made) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "slab split: " + why};
-  if (!(flags & kFlagCallerWorkspace))
+  if (!(flags & DFFT_FLAG_CALLER_WORKSPACE))
     cuda_check(cudaMalloc(&P->work, P->work_bytes), "cudaMalloc(workspace)");
   return P.release();
 }

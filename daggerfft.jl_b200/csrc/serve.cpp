@@ -197,7 +197,7 @@ static void CUDART_CB on_done(void* p) {
   s->srv->poke();
 }
 
-// Server plans own no workspace (kFlagCallerWorkspace): while it runs a
+// Server plans own no workspace (DFFT_FLAG_CALLER_WORKSPACE): while it runs a
 // plan only reads its tables, and each request brings its workspace (C2R
 // scratch, Bluestein scratch, fused-pass counters) from the arena, so one
 // resident instance serves every concurrent request of its shape.  Called
@@ -217,7 +217,7 @@ static Plan* get_plan(Server* S, const PlanKey& k, const dfft_request& r) {
   }
   std::unique_ptr<Plan> p(build_plan(r.ndim, r.shape, r.precision, r.transform, r.ndims, r.dims, r.r2r_kinds,
                                      r.irfft_len, r.decomp, DFFT_PLAIN,
-                                     (S->flags & DFFT_FLAG_TUNE) | kFlagCallerWorkspace));
+                                     (S->flags & DFFT_FLAG_TUNE) | DFFT_FLAG_CALLER_WORKSPACE));
   std::lock_guard<std::mutex> lk(S->mu);
   S->all_plans.push_back(p.get());
   S->shared_plans[k] = p.get();

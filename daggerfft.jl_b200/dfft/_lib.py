@@ -36,6 +36,7 @@ FLAG_TUNE = 1 << 1
 FLAG_NO_WISDOM = 1 << 2
 FLAG_NO_FUSE = 1 << 3
 FLAG_FUSE = 1 << 4
+FLAG_CALLER_WORKSPACE = 1 << 5
 
 
 class DFFTError(RuntimeError):
@@ -82,6 +83,8 @@ def lib():
     L.dfft_plan_describe.restype = c_int
     L.dfft_execute.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p]
     L.dfft_execute.restype = c_int
+    L.dfft_execute_workspace.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
+    L.dfft_execute_workspace.restype = c_int
     L.dfft_plan_destroy.argtypes = [c_void_p]
     L.dfft_plan_destroy.restype = c_int
     L.dfft_device_error.argtypes = [ctypes.POINTER(c_int)]

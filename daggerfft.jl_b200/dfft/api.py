@@ -246,6 +246,8 @@ class Plan:
         wb = ctypes.c_size_t()
         check(L.dfft_plan_workspace_bytes(h, ctypes.byref(wb)))
         self.workspace_bytes = wb.value
+        # bytes an execution brings itself (0: the plan's own workspace serves it)
+        self._bring = wb.value if int(flags) & _lib.FLAG_CALLER_WORKSPACE else 0
         self._out_strides = _strides(self.out_shape, order)
 
     def describe(self) -> str:
@@ -260,7 +262,18 @@ class Plan:
             s = _stream_handle(inp.device.index)
         else:
             s = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream or 0)
-        st = self._L.dfft_execute(self._h, inp.data_ptr(), out.data_ptr(), s)
+        if self._bring:
+            # this execution's own workspace, from torch's allocator on the same
+            # stream: reused only after the passes enqueued here
+            if stream is None:
+                w = torch.empty(self._bring, dtype=torch.uint8, device=inp.device)
+                st = self._L.dfft_execute_workspace(self._h, inp.data_ptr(), out.data_ptr(), s, w.data_ptr())
+            else:
+                w = torch.cuda.caching_allocator_alloc(self._bring, inp.device, s)
+                st = self._L.dfft_execute_workspace(self._h, inp.data_ptr(), out.data_ptr(), s, w)
+                torch.cuda.caching_allocator_delete(w)
+        else:
+            st = self._L.dfft_execute(self._h, inp.data_ptr(), out.data_ptr(), s)
         if st:
             check(st)
         return out
@@ -295,7 +308,8 @@ def _new_plan(transform, A, o, dims, n, decomp, method, flags):
 def get_or_create_gpu_plan(transform, A: torch.Tensor, dims, n=None, decomp=None,
                            method="plain", flags=0) -> Plan:
     """src/fftgpu.jl:107-116; key (eltype, size, tag, dims) plus the layout,
-    device, real length, decomposition and arithmetic form."""
+    device, real length, decomposition and arithmetic form.  The plan holds
+    its workspace: execute it on one stream at a time."""
     if not isinstance(transform, Transform):
         raise ArgumentError(_lib.ERROR_UNKNOWN_TRANSFORM, "Unknown transform type")
     return _cached_plan(transform, A, _order(A), dims, n, decomp, method, flags)
@@ -307,10 +321,21 @@ def _cached_plan(transform, A, o, dims, n, decomp, method, flags):
            method, flags, A.device.index)
     p = GPU_PLAN_CACHE.get(key)
     if p is None:
-        p = _new_plan(transform, A, o, dims_t, n, decomp, method, flags)
+        # a plan without workspace is the same with either of the two flags
+        twin = GPU_PLAN_CACHE.get(key[:8] + (flags ^ _lib.FLAG_CALLER_WORKSPACE,) + key[9:])
+        p = twin if twin is not None and twin.workspace_bytes == 0 else \
+            _new_plan(transform, A, o, dims_t, n, decomp, method, flags)
         with _CACHE_LOCK:
             p = GPU_PLAN_CACHE.setdefault(key, p)
     return p
+
+
+def _call_plan(transform, A, o, dims, n=None, decomp=None, method="plain", flags=0):
+    """The plan behind a call whose caller never sees it (``fft`` and the other
+    functions here, the distributed-array stages).  It holds no workspace, each
+    execution brings its own: such calls may run on several streams or threads
+    at once, and a plan's job counters or intermediate arrays must not meet."""
+    return _cached_plan(transform, A, o, dims, n, decomp, method, flags | _lib.FLAG_CALLER_WORKSPACE)
 
 
 def gpu_cleanup_plans():
@@ -328,7 +353,9 @@ def apply_gpu_fft_(out: torch.Tensor, inp: torch.Tensor, transform, dim, n=None,
                    method="plain"):
     """``apply_gpu_fft!(out, in, transform, dim)``: plan lookup + ``mul!``."""
     _check_tensor(inp)
-    p = get_or_create_gpu_plan(transform, inp, dim, n, decomp, method)
+    if not isinstance(transform, Transform):
+        raise ArgumentError(_lib.ERROR_UNKNOWN_TRANSFORM, "Unknown transform type")
+    p = _call_plan(transform, inp, _order(inp), dim, n, decomp, method)
     if tuple(out.shape) != p.out_shape:
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, f"output shape {tuple(out.shape)} != {p.out_shape}")
     if _order(out) != _order(inp) and out.dim() > 1:
@@ -353,7 +380,7 @@ def _run(transform, A, dims, n=None, decomp=None, method="plain", flags=0, out_d
     o = _order(A)
     if o == "X":
         A, o = A.contiguous(), "C"
-    p = _cached_plan(transform, A, o, dims, n, decomp, method, flags)
+    p = _call_plan(transform, A, o, dims, n, decomp, method, flags)
     out = torch.empty_strided(p.out_shape, p._out_strides, dtype=out_dtype or A.dtype, device=A.device)
     return p.execute(A, out)
 
@@ -429,7 +456,7 @@ def fft_(A, decomp=None, dims=(1, 2, 3), method="plain"):
     A_ = _prep(A)
     if A_.data_ptr() != A.data_ptr():
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, "fft! needs a contiguous array")
-    p = get_or_create_gpu_plan(FFT_(), A, _norm_dims(dims, A.dim()), decomp=decomp, method=method)
+    p = _call_plan(FFT_(), A, _order(A), _norm_dims(dims, A.dim()), decomp=decomp, method=method)
     return p.execute(A, A)
 
 
@@ -438,7 +465,7 @@ def ifft_(A, decomp=None, dims=(1, 2, 3), method="plain"):
     A_ = _prep(A)
     if A_.data_ptr() != A.data_ptr():
         raise ArgumentError(_lib.ERROR_INVALID_VALUE, "ifft! needs a contiguous array")
-    p = get_or_create_gpu_plan(IFFT_(), A, _norm_dims(dims, A.dim()), decomp=decomp, method=method)
+    p = _call_plan(IFFT_(), A, _order(A), _norm_dims(dims, A.dim()), decomp=decomp, method=method)
     return p.execute(A, A)
 
 

@@ -33,8 +33,8 @@ import torch
 
 from . import _lib
 from ._lib import ArgumentError, check
-from .api import (FFT, FFT_, IFFT, IFFT_, Pencil, Slab, Transform, _order,
-                  get_or_create_gpu_plan)
+from .api import (FFT, FFT_, IFFT, IFFT_, Pencil, Slab, Transform, _call_plan,
+                  _order)
 
 Range3 = Tuple[range, range, range]
 
@@ -362,7 +362,7 @@ def gpu_coalesced_redistribute_(dst: DArray, src: DArray, ws: Workspace, phase_i
 def _stage(D: DArray, transform, dims):
     for i in D.local_indices:
         c = D.chunks[i]
-        p = get_or_create_gpu_plan(transform, c, dims)
+        p = _call_plan(transform, c, _order(c), dims)
         p.execute(c, c)
 
 

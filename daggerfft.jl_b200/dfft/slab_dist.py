@@ -41,7 +41,7 @@ import torch
 
 from . import _lib
 from ._lib import ArgumentError, check
-from .api import FFT_, IFFT_, _precision, get_or_create_gpu_plan
+from .api import FFT_, IFFT_, _call_plan, _order, _precision
 
 
 def zsplit(n3: int, world: int) -> List[Tuple[int, int]]:
@@ -154,7 +154,7 @@ class CudaSlabKernels:
 
     def zpass(self, B: torch.Tensor, inverse: bool):
         t = IFFT_() if inverse else FFT_()
-        p = get_or_create_gpu_plan(t, B, (3,))
+        p = _call_plan(t, B, _order(B), (3,))
         p.execute(B, B)
 
     def copy(self, dst: torch.Tensor, src: torch.Tensor):

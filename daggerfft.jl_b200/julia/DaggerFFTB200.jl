@@ -62,8 +62,9 @@ end
 mutable struct Plan
     h::Ptr{Cvoid}
     outsize::Tuple
-    function Plan(h, outsize)
-        p = new(h, outsize)
+    ws::Int   # bytes of workspace every execution brings (0: the plan holds its own)
+    function Plan(h, outsize, ws=0)
+        p = new(h, outsize, ws)
         finalizer(p) do q
             q.h != C_NULL && ccall((:dfft_plan_destroy, libdfft), Cint, (Ptr{Cvoid},), q.h)
             q.h = C_NULL
@@ -74,6 +75,7 @@ end
 
 # plan cache keyed like GPU_PLAN_CACHE (src/fftgpu.jl:83-116)
 const GPU_PLAN_CACHE = Dict{Any,Plan}()
+const FLAG_CALLER_WORKSPACE = 1 << 5
 
 function plan_transform(transform, A::CuArray, dims; decomp=Pencil(), n=0, method=:plain, flags=0)
     dims_t = dims isa Tuple ? dims : (dims,)
@@ -90,9 +92,18 @@ function plan_transform(transform, A::CuArray, dims; decomp=Pencil(), n=0, metho
                     kinds, Int64(n), code(decomp), method_code(method), Cuint(flags)))
         out = zeros(Int64, ndims(A))
         check(ccall((:dfft_plan_output_shape, libdfft), Cint, (Ptr{Cvoid}, Ptr{Int64}), h[], out))
-        Plan(h[], Tuple(out))
+        ws = Ref{Csize_t}(0)
+        if flags & FLAG_CALLER_WORKSPACE != 0
+            check(ccall((:dfft_plan_workspace_bytes, libdfft), Cint, (Ptr{Cvoid}, Ref{Csize_t}), h[], ws))
+        end
+        Plan(h[], Tuple(out), Int(ws[]))
     end
 end
+
+# The plan behind a call whose caller never sees it: it holds no workspace,
+# each execution brings its own, so tasks (each on its own stream) share it.
+call_plan(transform, A::CuArray, dims; flags=0, kw...) =
+    plan_transform(transform, A, dims; flags=flags | FLAG_CALLER_WORKSPACE, kw...)
 
 "One line per kernel launch of a plan (`dfft_plan_describe`)."
 function describe(p::Plan)
@@ -102,6 +113,14 @@ function describe(p::Plan)
 end
 
 function execute!(p::Plan, out::CuArray, in::CuArray)
+    if p.ws > 0
+        ws = CuArray{UInt8}(undef, p.ws)   # freed in stream order below
+        check(ccall((:dfft_execute_workspace, libdfft), Cint,
+                    (Ptr{Cvoid}, CuPtr{Cvoid}, CuPtr{Cvoid}, Ptr{Cvoid}, CuPtr{Cvoid}),
+                    p.h, in, out, CUDA.stream().handle, ws))
+        CUDA.unsafe_free!(ws)
+        return out
+    end
     check(ccall((:dfft_execute, libdfft), Cint, (Ptr{Cvoid}, CuPtr{Cvoid}, CuPtr{Cvoid}, Ptr{Cvoid}),
                 p.h, in, out, CUDA.stream().handle))
     out
@@ -141,7 +160,7 @@ end
 
 "`apply_gpu_fft!(out, in, transform, dim)`: plan lookup + execute (src/fftgpu.jl:118-124)."
 function apply_gpu_fft!(out, in, transform, dim; kw...)
-    execute!(plan_transform(transform, in, dim; kw...), out, in)
+    execute!(call_plan(transform, in, dim; kw...), out, in)
 end
 
 cplx(::Type{Float32}) = ComplexF32
@@ -151,44 +170,44 @@ realt(::Type{ComplexF64}) = Float64
 
 function fft(A::CuArray; decomp=Pencil(), dims=(1, 2, 3), transforms=nothing, method=:plain)
     if transforms !== nothing && first(transforms) isa R2R
-        p = plan_transform(first(transforms), A, dims; decomp)
+        p = call_plan(first(transforms), A, dims; decomp)
         return execute!(p, similar(A, p.outsize), A)
     end
     B = eltype(A) <: Complex ? A : CuArray{cplx(eltype(A))}(A)
-    p = plan_transform(FFT(), B, dims; decomp, method)
+    p = call_plan(FFT(), B, dims; decomp, method)
     execute!(p, similar(B, p.outsize), B)
 end
 
 function ifft(A::CuArray; decomp=Pencil(), dims=(1, 2, 3), transforms=nothing, method=:plain)
     if transforms !== nothing && first(transforms) isa R2R
-        p = plan_transform(first(transforms), A, dims; decomp)
+        p = call_plan(first(transforms), A, dims; decomp)
         return execute!(p, similar(A, p.outsize), A)
     end
-    p = plan_transform(IFFT(), A, dims; decomp, method)
+    p = call_plan(IFFT(), A, dims; decomp, method)
     execute!(p, similar(A, p.outsize), A)
 end
 
 "In-place `fft!(A; decomp, dims, transforms, method)`: `A` is overwritten with its transform."
 function fft!(A::CuArray{<:Complex}; decomp=Pencil(), dims=(1, 2, 3), transforms=nothing, method=:plain)
     t = (transforms !== nothing && first(transforms) isa R2R) ? first(transforms) : FFT!()
-    execute!(plan_transform(t, A, dims; decomp, method), A, A)
+    execute!(call_plan(t, A, dims; decomp, method), A, A)
 end
 function fft!(A::CuArray{<:Real}; decomp=Pencil(), dims=(1, 2, 3), transforms)
-    execute!(plan_transform(first(transforms), A, dims; decomp), A, A)
+    execute!(call_plan(first(transforms), A, dims; decomp), A, A)
 end
 
 "In-place `ifft!(A; decomp, dims, method)` (scaled by 1/prod(size(A, dims)))."
 function ifft!(A::CuArray{<:Complex}; decomp=Pencil(), dims=(1, 2, 3), method=:plain)
-    execute!(plan_transform(IFFT!(), A, dims; decomp, method), A, A)
+    execute!(call_plan(IFFT!(), A, dims; decomp, method), A, A)
 end
 
 function rfft(A::CuArray{<:Real}; decomp=Pencil(), dims=(1, 2, 3))
-    p = plan_transform(RFFT(), A, dims; decomp)
+    p = call_plan(RFFT(), A, dims; decomp)
     execute!(p, CuArray{cplx(eltype(A))}(undef, p.outsize), A)
 end
 
 function irfft(F::CuArray{<:Complex}, d::Integer; decomp=Pencil(), dims=(1, 2, 3))
-    p = plan_transform(IRFFT(), F, dims; decomp, n=d)
+    p = call_plan(IRFFT(), F, dims; decomp, n=d)
     execute!(p, CuArray{realt(eltype(F))}(undef, p.outsize), F)
 end
 
@@ -578,7 +597,7 @@ end
 function stage!(D::ChunkedArray, transform, dims; method=:plain)
     for c in D.chunks
         c === nothing && continue
-        execute!(plan_transform(transform, c, dims; method), c, c)
+        execute!(call_plan(transform, c, dims; method), c, c)
     end
 end
 inplace(::Union{FFT,FFT!}) = FFT!()
@@ -694,7 +713,7 @@ function fused_slab_fft!(Bloc::CuArray{T,3}, Aloc::CuArray{T,3}, L::Integer, n3:
         end
     end
     isempty(reqs) || mpi.Waitall(mpi.RequestSet(reqs))
-    execute!(plan_transform(FFT!(), Bloc, (3,)), Bloc, Bloc)
+    execute!(call_plan(FFT!(), Bloc, (3,)), Bloc, Bloc)
     Bloc
 end
 
@@ -715,7 +734,7 @@ function fused_slab_ifft!(Aloc::CuArray{T,3}, Bloc::CuArray{T,3}, L::Integer, n3
     groups = [slab_groups(zs[s+1][2], ngroups) for s in 1:nranks]
     buf = CuArray{T}(undef, LR * Zr * nranks)
     Bv = vec(Bloc)
-    execute!(plan_transform(IFFT!(), Bloc, (3,)), Bloc, Bloc)
+    execute!(call_plan(IFFT!(), Bloc, (3,)), Bloc, Bloc)
     CUDA.synchronize()
     mpi = comm === nothing ? nothing :
           Base.require(Base.PkgId(Base.UUID("da04e1cc-30fd-572f-bb4f-1f8673147195"), "MPI"))

@@ -21,7 +21,9 @@
  *     FIRST transformed dim to n/2+1; irfft needs the real length d; r2r
  *     kinds are FFTW's and unnormalised.
  *   - Threading: a plan may be used by one stream at a time; distinct plans
- *     may be used concurrently from any thread.
+ *     may be used concurrently from any thread.  Executions that bring their
+ *     own workspace (dfft_execute_workspace) share nothing but the plan's
+ *     tables: one plan then serves any number of streams and threads.
  */
 #ifndef DFFT_H
 #define DFFT_H
@@ -93,8 +95,11 @@ enum {
   DFFT_FLAG_NO_WISDOM = 1u << 2,     /* ignore the tuning cache              */
   DFFT_FLAG_NO_FUSE = 1u << 3,       /* one pass per axis: no fused 2-D slab
                                         pass over dims (1, 2)                */
-  DFFT_FLAG_FUSE = 1u << 4           /* use the fused slab pass wherever a
+  DFFT_FLAG_FUSE = 1u << 4,          /* use the fused slab pass wherever a
                                         kernel exists (no timing)            */
+  DFFT_FLAG_CALLER_WORKSPACE = 1u << 5 /* the plan holds no workspace: every
+                                        execution brings its own
+                                        (dfft_execute_workspace)             */
 };
 
 typedef struct dfft_plan_s* dfft_plan;
@@ -148,7 +153,8 @@ DFFT_API int dfft_slab_split_create(dfft_plan* plan, int precision, int inverse,
 /* Output shape (column-major, ndim entries) of a plan. */
 DFFT_API int dfft_plan_output_shape(dfft_plan plan, int64_t* shape);
 
-/* Device workspace the plan holds (bytes, twiddles excluded). */
+/* Device workspace the plan holds, or with DFFT_FLAG_CALLER_WORKSPACE needs
+ * at every execution (bytes, twiddles excluded). */
 DFFT_API int dfft_plan_workspace_bytes(dfft_plan plan, size_t* bytes);
 
 /* Number of kernel launches one dfft_execute makes. */
@@ -168,6 +174,16 @@ DFFT_API int dfft_plan_describe(dfft_plan plan, char* buf, size_t len);
  * in == out is allowed for C2C and R2R (in-place).
  */
 DFFT_API int dfft_execute(dfft_plan plan, const void* in, void* out, void* stream);
+
+/*
+ * The same with the workspace of this execution supplied by the caller
+ * (dfft_plan_workspace_bytes bytes, 256-byte aligned, contents arbitrary; may
+ * be NULL when that is 0): intermediate arrays and the job counters of the
+ * fused slab pass live there, so concurrent executions of one plan on
+ * different streams do not meet.  The workspace must stay untouched until the
+ * execution is complete in stream order.
+ */
+DFFT_API int dfft_execute_workspace(dfft_plan plan, const void* in, void* out, void* stream, void* workspace);
 
 /* Release a plan (gpu_cleanup_workspace!, src/fftgpu.jl:630-634). */
 DFFT_API int dfft_plan_destroy(dfft_plan plan);
