@@ -133,6 +133,13 @@ __device__ __forceinline__ WholeAxis whole_axis(const IoAny& io, long long b) {
   return WholeAxis{b - j * io.t_i, io.t_i, (int)j, io.t_m};
 }
 
+// Do the real pairs of a column with unit stride sit on whole complex elements
+// (one access per pair)?  An offset view of a larger real array is only
+// aligned to its own type.
+template <typename T> __device__ __forceinline__ bool whole_pairs(const T* first) {
+  return (reinterpret_cast<uintptr_t>(first) & (2 * sizeof(T) - 1)) == 0;
+}
+
 // Base of column q on side io.
 __device__ __forceinline__ long long column_base(const IoAny& io, long long I, long long q) {
   const long long qo = I == 1 ? q : q / I;
@@ -172,7 +179,7 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
         in([=](int k) { return pc[b + k * sk]; });
         break;
       case IO_REAL_PAIR:
-        if (sk == 1) in([=](int k) { return *reinterpret_cast<const V*>(pr + b + 2 * (long long)k); });
+        if (sk == 1 && whole_pairs(pr + b)) in([=](int k) { return *reinterpret_cast<const V*>(pr + b + 2 * (long long)k); });
         else in([=](int k) { return mk<V>(pr[b + (2 * k) * sk], pr[b + (2 * k + 1) * sk]); });
         break;
       case IO_REAL:
@@ -269,7 +276,7 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
         break;
       }
       case IO_REAL_PAIR:
-        if (sk == 1) out(L, [=](int k, V v) { *reinterpret_cast<V*>(pr + b + 2 * (long long)k) = cscale(v, s); });
+        if (sk == 1 && whole_pairs(pr + b)) out(L, [=](int k, V v) { *reinterpret_cast<V*>(pr + b + 2 * (long long)k) = cscale(v, s); });
         else out(L, [=](int k, V v) {
           pr[b + (2 * k) * sk] = v.x * s;
           pr[b + (2 * k + 1) * sk] = v.y * s;

@@ -146,6 +146,7 @@ void execute_batch(Batch* B, const void* const* ins, void* const* outs, cudaStre
   const int n = (int)B->plans.size();
   for (int i = 0; i < n; ++i)
     if (!ins[i] || !outs[i]) throw Error{DFFT_ERROR_INVALID_VALUE, "NULL buffer in batch"};
+  for (int i = 0; i < n; ++i) check_alignment(B->plans[i], ins[i], outs[i]);
   int cur = -1;
   cuda_check(cudaGetDevice(&cur), "cudaGetDevice");
   if (cur != B->device) cuda_check(cudaSetDevice(B->device), "cudaSetDevice");

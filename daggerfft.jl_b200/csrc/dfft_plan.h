@@ -39,6 +39,10 @@ Plan* build_plan(int ndim, const int64_t* shape, int precision, int transform, i
 Plan* build_slab_split_plan(int precision, int inverse, int64_t L, int64_t nslab, int64_t zr, int nranks,
                             int split_dim, unsigned flags);
 
+// Throws unless in and out are aligned to the elements of the plan's arrays
+// (every kernel moves whole ones; an address between them would fault).
+void check_alignment(const Plan* p, const void* in, const void* out);
+
 // work / chirp: workspaces supplied by the caller for this execution (null:
 // the plan's own); a plan built with DFFT_FLAG_CALLER_WORKSPACE owns none.
 // overlap: the launches may overlap the tails of the kernels before them.

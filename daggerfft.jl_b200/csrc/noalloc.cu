@@ -198,6 +198,10 @@ extern "C" int dfft_irfft_noalloc_f32(const void* in, void* out, int ndim, const
     set_error("irfft_noalloc: NULL argument or ndim outside 1..3");
     return DFFT_ERROR_INVALID_VALUE;
   }
+  if (reinterpret_cast<uintptr_t>(in) % sizeof(float2) || reinterpret_cast<uintptr_t>(out) % sizeof(float)) {
+    set_error("irfft_noalloc: array not aligned to its elements");
+    return DFFT_ERROR_INVALID_VALUE;
+  }
   long long R[3] = {1, 1, 1};
   for (int i = 0; i < ndim; ++i) {
     if (shape[i] < 1 || shape[i] > 0x7fffffffLL) {

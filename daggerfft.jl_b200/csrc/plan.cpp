@@ -384,9 +384,16 @@ Plan::~Plan() {
 size_t Plan::in_bytes() const { return (size_t)(in_shape[0] * in_shape[1] * in_shape[2]) * in_elem; }
 size_t Plan::out_bytes() const { return (size_t)(out_shape[0] * out_shape[1] * out_shape[2]) * out_elem; }
 
+void check_alignment(const Plan* P, const void* in, const void* out) {
+  if (P->passes.empty()) return;  // a copy
+  if (reinterpret_cast<uintptr_t>(in) % P->in_elem || reinterpret_cast<uintptr_t>(out) % P->out_elem)
+    cuda_check(cudaErrorMisalignedAddress, "array not aligned to its elements");
+}
+
 void execute_plan(const Plan* P, const void* in, void* out, cudaStream_t stream, void* work, void* chirp,
                   bool overlap) {
   if (!in || !out) throw Error{DFFT_ERROR_INVALID_VALUE, "in/out is NULL"};
+  check_alignment(P, in, out);
   if (!work) work = P->work;
   if (!chirp) chirp = P->chirp;
   if ((P->work_bytes && !work) || (P->chirp_bytes && !chirp))

@@ -1,0 +1,76 @@
+"""Arrays that start in the middle of a larger buffer: a contiguous view at an
+odd element offset is aligned to its own type only.  Real sides read and
+write pairs of such a view element by element; a complex address that is not
+a multiple of the element size is an error status, before any launch."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import dfft
+import dfft_oracle as oracle
+from dfft import _lib
+from helpers import rand, rel, to_np, tol_for
+
+pytestmark = pytest.mark.gpu
+
+
+def offset_view(a, order="F", skip=1):
+    """Device copy of `a` whose first element is `skip` elements into its buffer."""
+    flat = np.concatenate([np.zeros(skip, a.dtype), a.ravel(order=order)])
+    t = torch.from_numpy(flat).cuda()[skip:]
+    assert t.data_ptr() % (2 * a.itemsize) == (skip % 2) * a.itemsize
+    if order == "C":
+        return t.view(a.shape)
+    return t.view(tuple(reversed(a.shape))).permute(*reversed(range(a.ndim)))
+
+
+@pytest.mark.parametrize("shape,dims", [((1000, 3), (1,)), ((250, 7), (1,)), ((20, 22, 5), (1, 2, 3)), ((74, 5), (1,)),
+                                        ((40002, 2), (1,)), ((6, 250), (2,))])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_rfft_and_irfft_of_offset_views(shape, dims, dtype):
+    a = rand(shape, dtype, seed=shape[0])
+    x = offset_view(a)
+    ref = oracle.rfft(a, dims=dims)
+    F = dfft.rfft(x, dims=dims)
+    assert rel(to_np(F), ref) <= tol_for(dtype)
+    n = shape[dims[0] - 1]
+    p = dfft.gpu_plan_transform(dfft.IRFFT(), F, dims, n=n)
+    out = offset_view(np.zeros_like(a))
+    p.execute(F, out)
+    assert rel(to_np(out), a) <= tol_for(dtype)
+
+
+@pytest.mark.parametrize("dtype,off", [(torch.complex64, 4), (torch.complex128, 8)])
+@pytest.mark.parametrize("n", [64, 251, 1200, 5000, 1 << 17])
+def test_complex_address_between_elements_is_refused(dtype, off, n):
+    x = torch.zeros(2 * n + 2, dtype=dtype, device="cuda")
+    p = dfft.gpu_plan_transform(dfft.FFT(), x[:n], (1,))
+    L = dfft.lib()
+    a, b = x.data_ptr(), x[n + 1:].data_ptr()
+    for i, o in ((a + off, b), (a, b + off)):
+        assert L.dfft_execute(p._h, i, o, 0) == _lib.ERROR_CUDA
+    for persistent in (False, True):
+        batch = dfft.Batch([p], persistent=persistent)
+        ins, outs = (ctypes.c_void_p * 1)(a + off), (ctypes.c_void_p * 1)(b)
+        assert L.dfft_batch_execute(batch._h, ins, outs, None) == _lib.ERROR_CUDA
+    torch.cuda.synchronize()
+    assert float(x.abs().sum()) == 0
+    p.execute(x[:n], x[n:2 * n])
+    torch.cuda.synchronize()
+
+
+def test_no_alloc_entry_point_on_offset_arrays():
+    f = dfft.lib().dfft_irfft_noalloc_f32
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
+                                           ctypes.POINTER(ctypes.c_int64), ctypes.c_void_p]
+    a = rand((250, 6), np.float32, seed=3)
+    F = torch.from_numpy(np.ascontiguousarray(oracle.rfft(a, dims=(1,)).T.astype(np.complex64))).cuda()
+    out = offset_view(np.zeros_like(a))
+    shape = (ctypes.c_int64 * 2)(250, 6)
+    assert f(F.data_ptr() + 4, out.data_ptr(), 2, shape, None) == _lib.ERROR_INVALID_VALUE
+    ref = to_np(dfft.irfft(F.permute(1, 0), 250, dims=(1, 2)))
+    assert f(F.data_ptr(), out.data_ptr(), 2, shape, None) == 0
+    torch.cuda.synchronize()
+    assert rel(to_np(out), ref) <= 1e-5
