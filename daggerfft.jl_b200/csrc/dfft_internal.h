@@ -48,6 +48,7 @@ struct Pass {
   size_t src_off = 0, dst_off = 0;  // byte offsets into those buffers
   bool is_static = false;
   int dbl = 0;  // precision
+  std::shared_ptr<const Pass> unaligned;  // launched instead for arrays not 16-byte aligned (null: refused)
   int four_step = 0;  // 1, 2: first / second pass of a four-step axis
   bool fsfirst = false;  // four_step_first
   FourStepGeom fsgeom{};

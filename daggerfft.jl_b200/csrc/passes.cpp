@@ -667,7 +667,13 @@ Pass make_pass(const PassSpec& s) {
   if (s.variant == VARIANT_ASYNC) return make_async_pass(s);
   if (s.variant == VARIANT_AUTO && tiled_kind(s)) {
     try {
-      return make_tiled_pass(s);
+      Pass p = make_tiled_pass(s);
+      // bulk copies start on 16 bytes; real arrays at any element (a view at
+      // an odd offset of a larger one) run the one-tile kernel
+      PassSpec t = s;
+      t.variant = VARIANT_DIRECT;
+      p.unaligned = std::make_shared<const Pass>(make_pass(t));
+      return p;
     } catch (const Error& e) {
       if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
     }
@@ -1151,6 +1157,8 @@ static cudaError_t launch_serial(const Pass& p, void** args, cudaStream_t stream
 
 cudaError_t launch_pass(const Pass& p, void* in, void* out, cudaStream_t stream, void* work, bool overlap) {
   if (p.grid.x == 0) return cudaSuccess;
+  if (p.unaligned && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return launch_pass(*p.unaligned, in, out, stream, work, overlap);
   cudaError_t e = cudaSuccess;  // (the shared-memory limit is raised when the pass is made)
   PassDesc d = p.d;
   d.in.p = in;

@@ -74,3 +74,23 @@ def test_no_alloc_entry_point_on_offset_arrays():
     assert f(F.data_ptr(), out.data_ptr(), 2, shape, None) == 0
     torch.cuda.synchronize()
     assert rel(to_np(out), ref) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [128, 256, 512])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", [dfft.REDFT10, dfft.REDFT01])
+@pytest.mark.parametrize("cols,strided", [(1, False), (13, False), (16, False), (4, True), (16, True)])
+def test_dct_of_offset_views(n, dtype, kind, cols, strided):
+    shape, dims = ((cols, n, 3), (2,)) if strided else ((n, cols), (1,))
+    a = rand(shape, dtype, seed=n + cols)
+    x = offset_view(a)
+    tr = (dfft.R2R((kind,)),)
+    p = dfft.gpu_plan_transform(tr[0], x, dims)
+    assert p.describe().startswith("tiled"), p.describe()
+    ref = oracle.fft(a, dims=dims, transforms=(oracle.R2R((kind,)),))
+    assert rel(to_np(dfft.fft(x, dims=dims, transforms=tr)), ref) <= tol_for(dtype)  # input between 16 bytes
+    out = offset_view(np.zeros_like(a))
+    p.execute(offset_view(a, skip=0), out)
+    assert rel(to_np(out), ref) <= tol_for(dtype)  # output
+    p.execute(x, x)
+    assert rel(to_np(x), ref) <= tol_for(dtype)  # in place
