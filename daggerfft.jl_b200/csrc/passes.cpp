@@ -1492,6 +1492,12 @@ static void four_step_pair(const PassSpec& s, int L1, int L2, unsigned flags, Pa
       b.variant = VARIANT_AUTO;
       *pb = plan_pass(b, flags);
     }
+    // its output is the caller's array: the TMA kernels store on 16 bytes, an
+    // 8-byte aligned ComplexF32 array takes the one-tile kernel
+    PassSpec u = b;
+    u.variant = four_step_factor(s.dbl, L1);
+    u.C = 0;
+    pb->unaligned = std::make_shared<const Pass>(make_pass(u));
   } else {
     *pb = make_pass(b);
   }

@@ -95,3 +95,20 @@ def test_dct_of_offset_views(n, dtype, kind, cols, strided):
     assert rel(to_np(out), ref) <= tol_for(dtype)  # output
     p.execute(x, x)
     assert rel(to_np(x), ref) <= tol_for(dtype)  # in place
+
+
+@pytest.mark.parametrize("shape,dims", [((1 << 17,), (1,)), ((1 << 20,), (1,)), ((45000, 3), (1,)), ((3, 20480, 2), (2,)),
+                                        ((143 * 128, 2), (1,)), ((20011, 2), (1,)), ((2, 40009), (2,))])
+def test_long_axes_of_offset_views(shape, dims):
+    a = rand(shape, np.complex64, seed=len(shape))
+    x = offset_view(a)
+    ref = oracle.fft(a, dims=dims)
+    p = dfft.gpu_plan_transform(dfft.FFT(), x, dims)
+    assert "four-step" in p.describe(), p.describe()
+    out = offset_view(np.zeros_like(a))
+    p.execute(x, out)
+    assert rel(to_np(out), ref) <= tol_for(np.complex64)
+    dfft.fft_(x, dims=dims)
+    assert rel(to_np(x), ref) <= tol_for(np.complex64)
+    dfft.ifft_(x, dims=dims)
+    assert rel(to_np(x), a) <= tol_for(np.complex64)
