@@ -1071,7 +1071,6 @@ static Pass make_slab_cols_pass(int dbl, int L, long long nslab, int inverse, in
   g.rout = rout;
   g.zr = zr;
   const SlabKernel* k = find_slab_kernel(dbl, L, v);
-  if (!k->fn_cols) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "no rank-split slab kernel for this length"};
   p.fn = inverse ? k->fn_inv_cols : k->fn_cols;
   cuda_check(ensure_smem_attr(p.fn, p.smem), "cudaFuncSetAttribute(slab cols)");
   int occ = 0;
@@ -1117,7 +1116,6 @@ Pass make_slab_split_pass(int dbl, int L, long long nslab, int inverse, int v, i
   g.rout = rout;
   g.zr = zr;
   const SlabKernel* k = find_slab_kernel(dbl, L, v);
-  if (!k->fn_split) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "no rank-split slab kernel for this length"};
   p.fn = inverse ? k->fn_inv_split : k->fn_split;
   cuda_check(ensure_smem_attr(p.fn, p.smem), "cudaFuncSetAttribute(slab split)");
   int occ = 0;

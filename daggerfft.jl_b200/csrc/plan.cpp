@@ -350,7 +350,7 @@ Plan* build_slab_split_plan(int precision, int inverse, int64_t L, int64_t nslab
   bool made = false;
   std::string why = "no fused slab kernel for this length";
   for (int v = 0; const SlabKernel* k = find_slab_kernel(dbl, (int)L, v); ++v) {
-    if (!k->dflt) continue;
+    if (!k->dflt || !k->fn_split) continue;  // (192 and 384: plain layout only)
     try {
       Pass p = make_slab_split_pass(dbl, (int)L, nslab, inverse, v, rin, rout, zr, split_dim);
       p.src = BUF_IN;

@@ -195,3 +195,22 @@ def test_two_radix_lengths(L, O, dtype):
     q.execute(out, out)
     assert rel(to_np(out), a) <= tol
     assert dfft.device_error() == 0
+
+
+@pytest.mark.parametrize("L", [192, 384])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("split_dim", [1, 2])
+@pytest.mark.parametrize("nranks", [1, 2, 3])
+def test_rank_split_of_plain_only_lengths_is_unsupported(L, precision, split_dim, nranks):
+    # lengths whose slab kernels have no rank-split form report the size, at
+    # any rank count, as every length without a kernel does
+    import ctypes
+
+    from dfft import _lib
+    h = ctypes.c_void_p()
+    f = dfft.lib().dfft_slab_split_create
+    f.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int64,
+                  ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_uint]
+    for inverse in (0, 1):
+        assert f(ctypes.byref(h), precision, inverse, L, 2, 2, nranks, split_dim, 0) == _lib.ERROR_UNSUPPORTED_SIZE
+        assert not h.value
