@@ -268,9 +268,11 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
       }
       case IO_CPLX_TW: {
         const unsigned jj = (unsigned)((b % io.t_ia) / io.t_i);
+        const int sh = io.n;
+        const V* hi = w + (1 << sh);
         const auto twiddle = [=](int k) {
           const unsigned m = jj * (unsigned)k;
-          return cmul(ldg_c(w + m % kTwSplit), ldg_c(w + kTwSplit + m / kTwSplit));
+          return split_twiddle(ldg_c(w + (m & ((1u << sh) - 1))), hi + 2 * (m >> sh));
         };
         column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, twiddle, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
         break;

@@ -32,7 +32,8 @@ struct FourStepGeom {
   int chirp_n;
   int inverse;
   const void* tw;   // M entries exp(-2 pi i m / M)
-  const void* twl;  // split twiddle table of W_L (kTwSplit low entries, then the high ones)
+  const void* twl;  // split twiddle table of W_L
+  int tw_log;       // log2 of its split
 };
 
 template <typename V, int CS, int R0, int R1> struct FourStepTile {
@@ -61,7 +62,8 @@ __global__ void __launch_bounds__(CS* P, MINB)
   const int n1_0 = (blockIdx.x - o * g.tiles) * CS;
   const V* twl = reinterpret_cast<const V*>(g.twl);
   const V* tw = reinterpret_cast<const V*>(g.tw);
-  for (int i = tid; i < kTwSplit; i += CS * P) lo[i] = twl[i];
+  const int sh = g.tw_log;
+  for (int i = tid; i < 1 << sh; i += CS * P) lo[i] = twl[i];
   pass_entry();
   {
     const int c = tid % CS, j = tid / CS;
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(CS* P, MINB)
     const int n1 = n1_0 + c;
     const V* col = sm + c * Tile::LD;
     V* dst = out + o * g.out_o + (long long)n1 * M;
-    const V* hi = twl + kTwSplit;
+    const V* hi = twl + (1 << sh);
 #pragma unroll
     for (int b = 0; b < BB; ++b) {
       const int j = t + b * P;
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(CS* P, MINB)
       for (int r = 0; r < R1; ++r) {
         const unsigned k = j + r * R0, m = (unsigned)n1 * k;
         if (g.inverse) v[r].y = -v[r].y;
-        dst[k] = cmul(v[r], cmul(lo[m % kTwSplit], ldg_c(hi + m / kTwSplit)));
+        dst[k] = cmul(v[r], split_twiddle(lo[m & ((1u << sh) - 1)], hi + 2 * (m >> sh)));
       }
     }
   }

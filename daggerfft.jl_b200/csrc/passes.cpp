@@ -1357,6 +1357,13 @@ static bool four_step_fast(const PassSpec& s) {
   return s.I == 1 && s.in.kind == IO_CPLX && s.in.si == 1 && s.in.sk == 1;
 }
 
+// The split of a W_L table: |W_L^m - 1| <= 1/32 below it.
+static int split_log(long long L) {
+  int sh = 1;
+  while ((2 << sh) <= kTwSplit && (2LL << sh) * 201 <= L) ++sh;
+  return sh;
+}
+
 static Pass make_four_step_first(const PassSpec& s, int L1, const FourStepKernel* k, const void* twl) {
   Pass p;
   p.dbl = s.dbl;
@@ -1385,6 +1392,7 @@ static Pass make_four_step_first(const PassSpec& s, int L1, const FourStepKernel
   auto tw = twiddle_table(s.dbl, k->M, 1, 0, k->M, false);
   g.tw = tw->p;
   g.twl = twl;
+  g.tw_log = split_log((long long)L1 * k->M);
   p.tables.push_back(tw);
   for (auto& t : s.keep) p.tables.push_back(t);
   const long long nblk = (long long)g.tiles * s.O;
@@ -1396,22 +1404,49 @@ static Pass make_four_step_first(const PassSpec& s, int L1, const FourStepKernel
   return p;
 }
 
-// W_L^m for m < kTwSplit, then W_L^(kTwSplit m) for kTwSplit m < L
-// (conjugated for an inverse).
-static std::shared_ptr<DevTable> split_twiddles(int dbl, long long L, bool conj) {
-  const int hi = (int)((L + kTwSplit - 1) / kTwSplit);
-  const size_t esz = dbl ? 16 : 8;
-  auto lo_t = twiddle_table(dbl, L, 1, 0, kTwSplit, conj);
-  auto hi_t = twiddle_table(dbl, L, kTwSplit, 0, hi, conj);
+static std::shared_ptr<DevTable> upload(int dbl, const std::vector<long double>& re,
+                                        const std::vector<long double>& im) {
+  const size_t n = re.size(), esz = dbl ? 16 : 8;
+  std::vector<unsigned char> host(esz * (n ? n : 1));
+  for (size_t k = 0; k < n; ++k) {
+    if (dbl) { double v[2] = {(double)re[k], (double)im[k]}; std::memcpy(&host[esz * k], v, esz); }
+    else { float v[2] = {(float)re[k], (float)im[k]}; std::memcpy(&host[esz * k], v, esz); }
+  }
   auto t = std::make_shared<DevTable>();
   cuda_check(cudaGetDevice(&t->device), "cudaGetDevice");
-  t->bytes = esz * (size_t)(kTwSplit + hi);
-  cuda_check(cudaMalloc(&t->p, t->bytes), "cudaMalloc(four-step twiddles)");
-  cuda_check(cudaMemcpy(t->p, lo_t->p, esz * kTwSplit, cudaMemcpyDeviceToDevice), "cudaMemcpy(four-step twiddles)");
-  cuda_check(cudaMemcpy(static_cast<char*>(t->p) + esz * kTwSplit, hi_t->p, esz * hi, cudaMemcpyDeviceToDevice),
-             "cudaMemcpy(four-step twiddles)");
-  // device-to-device copies do not wait: the first execute may be on a stream of its own
-  cuda_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize(four-step twiddles)");
+  t->bytes = host.size();
+  cuda_check(cudaMalloc(&t->p, t->bytes), "cudaMalloc(bluestein)");
+  cuda_check(cudaMemcpy(t->p, host.data(), t->bytes, cudaMemcpyHostToDevice), "cudaMemcpy(bluestein)");
+  return t;
+}
+
+// Split twiddle table of W_L (conjugated for an inverse), see split_twiddle.
+static std::shared_ptr<DevTable> split_twiddles(int dbl, long long L, bool conj) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, long long, bool>, std::weak_ptr<DevTable>> cache;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lk(mu);
+  auto& slot = cache[std::make_tuple(dev, dbl, L, conj)];
+  if (auto sp = slot.lock()) return sp;
+  const int S = 1 << split_log(L);
+  const long long H = (L + S - 1) / S;
+  const long double step = 2.0L * acosl(-1.0L) / (long double)L, sgn = conj ? 1.0L : -1.0L;
+  std::vector<long double> re, im;
+  for (int m = 0; m < S; ++m) {
+    const long double a = step * m, h = sinl(a / 2);
+    re.push_back(-2 * h * h);
+    im.push_back(sgn * sinl(a));
+  }
+  for (long long m = 0; m < H; ++m) {
+    const long double a = step * (long double)(m * S), c = cosl(a), d = sgn * sinl(a);
+    re.push_back(c);
+    im.push_back(d);
+    re.push_back(c - (dbl ? (long double)(double)c : (long double)(float)c));
+    im.push_back(d - (dbl ? (long double)(double)d : (long double)(float)d));
+  }
+  auto t = upload(dbl, re, im);
+  slot = t;
   return t;
 }
 
@@ -1449,7 +1484,7 @@ static void four_step_pair(const PassSpec& s, int L1, int L2, unsigned flags, Pa
   a.out.so = s.I * L2;
   a.out.sk = s.I;
   a.out.w = tw->p;
-  a.out.n = (int)L;
+  a.out.n = split_log(L);
   a.out.t_i = s.I * L2;
   a.out.t_ia = s.I * L;
   a.keep.push_back(tw);
@@ -1591,22 +1626,6 @@ static int smooth5_at_least(int n) {
       while (r % p == 0) r /= p;
     if (r == 1) return m;
   }
-}
-
-static std::shared_ptr<DevTable> upload(int dbl, const std::vector<long double>& re,
-                                        const std::vector<long double>& im) {
-  const size_t n = re.size(), esz = dbl ? 16 : 8;
-  std::vector<unsigned char> host(esz * (n ? n : 1));
-  for (size_t k = 0; k < n; ++k) {
-    if (dbl) { double v[2] = {(double)re[k], (double)im[k]}; std::memcpy(&host[esz * k], v, esz); }
-    else { float v[2] = {(float)re[k], (float)im[k]}; std::memcpy(&host[esz * k], v, esz); }
-  }
-  auto t = std::make_shared<DevTable>();
-  cuda_check(cudaGetDevice(&t->device), "cudaGetDevice");
-  t->bytes = host.size();
-  cuda_check(cudaMalloc(&t->p, t->bytes), "cudaMalloc(bluestein)");
-  cuda_check(cudaMemcpy(t->p, host.data(), t->bytes, cudaMemcpyHostToDevice), "cudaMemcpy(bluestein)");
-  return t;
 }
 
 // Convolution length for an N-point axis: the shortest compiled one, else the

@@ -199,3 +199,34 @@ def test_prime_over_two_radix_first_pass(n, dtype):
     assert rel(to_np(F), oracle.fft(a, dims=(1,))) <= tol_for(dtype)
     _, B = _run(dfft.IFFT(), F, (1,))
     assert rel(to_np(B), a) <= tol_for(dtype)
+
+
+@pytest.mark.parametrize("shape,dim", [((1 << 20,), 1), ((143 * 128,), 1), ((1 << 22,), 1), ((3, 1 << 17), 2),
+                                       ((2, 45000), 2)])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_four_step_twiddles_are_as_exact_as_a_table(shape, dim, dtype):
+    # an impulse at n < L1 goes through the first pass as 1, takes the twiddle
+    # W_L^(n k), and reaches the outputs k < L2 without another rounding: they
+    # are the twiddles themselves.  One rounding at full size (1/2 unit in 1)
+    # plus three at 1/32 of it; the product of two rounded entries has three
+    # roundings at full size.
+    L = shape[dim - 1]
+    u = float(np.finfo(np.zeros(1, dtype).real.dtype).eps) / 2
+    row = (0,) * (dim - 1)
+    for inverse in (False, True):
+        worst = 0.0
+        for n in (1, 2, 7, 61, 89, 101):
+            a = np.zeros(shape, dtype)
+            a[row + (n,)] = L if inverse else 1
+            p, F = _run(dfft.IFFT() if inverse else dfft.FFT(), to_gpu(a), (dim,))
+            first = p.describe().splitlines()[0]
+            assert "four-step=1" in first, first
+            L2 = int(first.split(" L=")[1].split()[0])
+            assert n < L // L2
+            k = np.arange(L2)
+            ang = 2 * np.arccos(np.longdouble(-1)) * ((n * k) % L).astype(np.longdouble) / L
+            y = to_np(F)[row][:L2]
+            s = 1 if inverse else -1
+            worst = max(worst, float(np.abs(y.real - np.cos(ang)).max()), float(np.abs(y.imag - s * np.sin(ang)).max()))
+        # (1/L of a length that is no power of two: L/L rounds once more)
+        assert worst <= (0.5 + 4 / 32 + (1.0 if inverse and L & (L - 1) else 0)) * u, worst / u
