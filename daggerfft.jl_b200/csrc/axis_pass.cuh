@@ -274,7 +274,7 @@ template <typename V> struct StageTw {
   }
 };
 // The same table with the last stage's entries pre-multiplied by the
-// inverse's 1/L (exact for power-of-two L): the last stage of an inverse
+// inverse's 1/L as rounded to T (exact for power-of-two L): the last stage of an inverse
 // then scales only its r = 0 inputs, and the DFT carries the scale to every
 // output (linearity), instead of scaling every output.
 template <typename V> struct StageTwScaledLast : StageTw<V> {};

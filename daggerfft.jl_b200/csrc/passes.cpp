@@ -995,8 +995,14 @@ Pass make_slab_pass(int dbl, int L, long long O, int inverse, int v) {
   };
   fill(p.d, 1);
   fill(p.d2, L);
-  // the inverse kernels fold 1/L into the last stage's twiddles
-  auto stw = stage_twiddles(dbl, L, rad, inverse ? 1.0 / (double)L : 1.0);
+  // the inverse kernels fold 1/L into the last stage's twiddles: the rounded
+  // 1/L that the kernel multiplies the r = 0 inputs by (for 384 and 192, where
+  // it is not exact, one factor for all: relative error of dims (1, 2) of
+  // 384^2 ComplexF32 planes 1.54e-7 with 1/L itself in the table, 1.45e-7 with
+  // the rounded one, 1.46e-7 with every output scaled at the store, which
+  // costs 2.5 % of 384^3)
+  const double fold = dbl ? 1.0 / (double)L : (double)(float)(1.0 / (double)L);
+  auto stw = stage_twiddles(dbl, L, rad, inverse ? fold : 1.0);
   p.tables.push_back(stw);
   p.d.tw = stw->p;
   auto twl = twiddle_table(dbl, L, 1, 0, L, false);

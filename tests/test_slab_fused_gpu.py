@@ -214,3 +214,25 @@ def test_rank_split_of_plain_only_lengths_is_unsupported(L, precision, split_dim
     for inverse in (0, 1):
         assert f(ctypes.byref(h), precision, inverse, L, 2, 2, nranks, split_dim, 0) == _lib.ERROR_UNSUPPORTED_SIZE
         assert not h.value
+
+
+@pytest.mark.parametrize("L", [192, 384])
+def test_inverse_scale_is_one_factor(L):
+    # 1/L is not exact at these lengths: the fused inverse multiplies everything
+    # by the same rounded 1/L, as the per-axis passes do.  Their errors agree
+    # to the few per cent that other radices cost; factors rounded one by one
+    # make the fused one 3 to 5 per cent larger.
+    e = {}
+    for flag in (dfft.FLAG_FUSE, dfft.FLAG_NO_FUSE):
+        s = r = 0.0
+        for seed in range(6):
+            a = rand((L, L, 8), np.complex64, seed=100 * L + seed)
+            g = to_gpu(a)
+            p = dfft.gpu_plan_transform(dfft.IFFT(), g, (1, 2), flags=flag)
+            out = dfft.empty_like_layout(p.out_shape, g.dtype, g)
+            p.execute(g, out)
+            ref = np.fft.ifft2(a.astype(np.complex128), axes=(0, 1))
+            s += float((np.abs(to_np(out) - ref) ** 2).sum())
+            r += float((np.abs(ref) ** 2).sum())
+        e[flag] = (s / r) ** 0.5
+    assert e[dfft.FLAG_FUSE] <= 1.02 * e[dfft.FLAG_NO_FUSE], e
