@@ -1791,25 +1791,15 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
   }
   // the outer direction is in the tables; the inner FFT_M pair is forward
   // then inverse
+  const int sgn = s.inverse ? +1 : -1;
   int M = bluestein_length(s.dbl, L);
-  if (four_step_fast(s) && !find_chirp_any(s.dbl, 2 * L - 1)) {
-    // convolutions beyond one CTA: the smallest length that splits into the
-    // two-radix first pass and a compiled factor of at most 2048 (1000003
-    // ComplexF32 points: 109 us through 1024 x 2000, 174 us through 1350 x
-    // 1500, the smallest one)
-    for (int m = M, i = 0; i < 64 && m < M + M / 4; m = smooth5_at_least(m + 1), ++i) {
-      int m1 = 0, m2 = 0;
-      if (!four_step_split(s.dbl, m, true, L, L, &m1, &m2) || !find_four_step_kernel(s.dbl, m2) || m1 > 2048) continue;
-      M = m;
-      break;
-    }
-  }
-  const BluesteinTables bt = bluestein_tables(s.dbl, L, s.inverse ? +1 : -1, M);
   const size_t csz = s.dbl ? 16 : 8;
   // both FFT_M, the filter and the two chirp multiplies on one tile in
   // shared memory (kEpiChirp); 251 x 9800 ComplexF32 columns: two passes
-  // through a scratch of M-point columns took 102 us, this 85
-  {
+  // through a scratch of M-point columns took 102 us, this 85.  The
+  // run-time-radix kernel holds at most 16 points in each of 1024 threads.
+  if (M <= 16 * 1024) {
+    const BluesteinTables bt = bluestein_tables(s.dbl, L, sgn, M);
     PassSpec one = s;
     one.L = M;
     one.inverse = 0;
@@ -1831,6 +1821,19 @@ size_t add_axis_passes(std::vector<Pass>& out, const PassSpec& s, unsigned flags
       if (e.status != DFFT_ERROR_UNSUPPORTED_SIZE) throw;
     }
   }
+  if (four_step_fast(s)) {
+    // convolutions beyond one CTA: the smallest length that splits into the
+    // two-radix first pass and a compiled factor of at most 2048 (1000003
+    // ComplexF32 points: 109 us through 1024 x 2000, 174 us through 1350 x
+    // 1500, the smallest one)
+    for (int m = M, i = 0; i < 64 && m < M + M / 4; m = smooth5_at_least(m + 1), ++i) {
+      int m1 = 0, m2 = 0;
+      if (!four_step_split(s.dbl, m, true, L, L, &m1, &m2) || !find_four_step_kernel(s.dbl, m2) || m1 > 2048) continue;
+      M = m;
+      break;
+    }
+  }
+  const BluesteinTables bt = bluestein_tables(s.dbl, L, sgn, M);
   // FFT_M does not fit one CTA: each FFT_M as a four-step pair, through two
   // scratch halves: x * chirp -> S1 -> S2 (the spectrum), S2 * Bhat -> S1 ->
   // out * chirp.  The last pass's sub-axis index k2 < M2 must stay below L

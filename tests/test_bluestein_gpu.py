@@ -80,3 +80,23 @@ def test_in_place_and_infinities_stay_in_their_column():
     keep[0, 2] = False
     assert not np.isfinite(y[0, :, 2]).any()
     assert rel(y.transpose(0, 2, 1)[keep], np.asarray(ref).transpose(0, 2, 1)[keep]) <= 1e-5
+
+
+@pytest.mark.parametrize("n,dtype", [(2053, np.complex64), (5003, np.complex64), (6007, np.complex64),
+                                     (1031, np.complex128), (2503, np.complex128)])
+def test_one_launch_takes_the_shortest_convolution(n, dtype):
+    # beyond the compiled lengths the one-launch kernel runs the smallest
+    # 5-smooth length, not the longer one a four-step pair would split into
+    shortest = next(k for k in range(2 * n - 1, 4 * n) if _smooth5(k))
+    a = rand((n, 3), dtype, seed=n)
+    p = _one_launch(dfft.FFT(), to_gpu(a), (1,))
+    assert f" L={shortest} " in p.describe(), p.describe()
+    F = dfft.fft(to_gpu(a), dims=(1,))
+    assert rel(to_np(F), oracle.fft(a, dims=(1,))) <= tol_for(dtype)
+
+
+def _smooth5(k):
+    for q in (2, 3, 5):
+        while k % q == 0:
+            k //= q
+    return k == 1
