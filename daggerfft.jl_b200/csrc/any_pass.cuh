@@ -29,13 +29,18 @@ namespace dfft {
 // that consecutive lanes touch consecutive memory of that side.  Columns
 // side by side (cfast): one column per thread, elements nthreads / C apart.
 // Unit stride along the column (the contiguous axis, and the output of a
-// four-step axis's first pass): groups of G lanes walk whole columns.
+// four-step axis's first pass): the column's share of the threads walks it, or
+// groups of G lanes do where that is less than a warp (fft + ifft of one
+// column of 5003 ComplexF32 points: 405 us with 32 lanes at work, 153 with all;
+// 40 Float32 pencils of 1002 points, rfft + irfft: 48 us, 118 with the side maps inside the stages).
 struct TileLanes {
   int c, cstep, k, kstep;
 };
 __device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, const IoAny& io, int L) {
   const int tid = threadIdx.x, n = blockDim.x;
   if (d.cfast && io.sk != 1) return TileLanes{tid % d.C, d.C, tid / d.C, n / d.C};
+  const int share = n / d.C;
+  if (share >= 32) return TileLanes{tid / share, n / share, tid % share, share};
   int G = 1;
   while (G < 32 && G < L && G * 2 <= n) G *= 2;
   const int groups = n / G;  // a remainder of n mod G threads moves nothing

@@ -60,3 +60,18 @@ def test_irfft_length_mismatch():
     # d = 17 also has 17//2+1 == 9 entries: both 16 and 17 are accepted
     x = dfft.irfft(F, 17, dims=(1,))
     assert x.shape[0] == 17
+
+
+@pytest.mark.parametrize("n", [62, 250, 500, 1000, 1002, 2000, 4000, 4095, 8190])
+@pytest.mark.parametrize("cols", [1, 2, 5])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_few_contiguous_pencils(n, cols, dtype):
+    # every column's share of the threads moves it: shares below, at and above
+    # a warp, tiles with columns that do not exist
+    a = rand((n, cols), dtype, seed=n + cols)
+    F = dfft.rfft(to_gpu(a), dims=(1,))
+    assert rel(to_np(F), oracle.rfft(a, dims=(1,))) <= tol_for(dtype)
+    assert rel(to_np(dfft.irfft(F, n, dims=(1,))), a) <= tol_for(dtype)
+    y = dfft.fft(to_gpu(a), dims=(1,), transforms=(dfft.R2R((dfft.DHT,)),))
+    h = np.fft.fft(a.astype(np.complex128), axis=0)
+    assert rel(to_np(y), h.real - h.imag) <= tol_for(dtype)
