@@ -95,7 +95,7 @@ struct SlabKernel {
   int lb;   // threads per CTA
   int cs;   // pencils / columns per tile
   int nb;   // tile buffers
-  int dflt; // an untuned plan may pick this variant (2, fused slab: for arrays of 48 MB and more)
+  int dflt; // an untuned plan may pick this variant (2 and 3, fused slab: for large arrays, see choose_slab)
   const void* fn;      // forward
   const void* fn_inv;  // inverse
   const void* fn_split;      // forward, rows split by rank

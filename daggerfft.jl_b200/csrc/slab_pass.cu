@@ -85,9 +85,9 @@ static const SlabKernel kSlabKernels[] = {
     {0, 128, 8, 2, {16, 8}, 160, 16, 2, 0, K(float, 160, 6, 2, 128, 8, 16, 16, 8)},
     {0, 128, 8, 2, {16, 8}, 160, 16, 3, 0, K(float, 160, 4, 3, 128, 8, 16, 16, 8)},
     {0, 384, 16, 2, {24, 16}, 160, 8, 2, 2, K2(float, 160, 4, 2, 384, 16, 8, 24, 16)},
-    {0, 192, 16, 2, {12, 16}, 160, 8, 2, 2, K2(float, 160, 6, 2, 192, 16, 8, 12, 16)},
+    {0, 192, 16, 2, {12, 16}, 160, 8, 2, 3, K2(float, 160, 6, 2, 192, 16, 8, 12, 16)},
     {1, 384, 16, 2, {24, 16}, 96, 4, 2, 2, K2(double, 96, 4, 2, 384, 16, 4, 24, 16)},
-    {1, 192, 16, 2, {12, 16}, 96, 4, 2, 2, K2(double, 96, 6, 2, 192, 16, 4, 12, 16)},
+    {1, 192, 16, 2, {12, 16}, 96, 4, 2, 3, K2(double, 96, 6, 2, 192, 16, 4, 12, 16)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 2, 1, K(double, 160, 5, 2, 512, 64, 2, 8, 8, 8)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 2, 1, K(double, 160, 4, 2, 512, 64, 2, 8, 8, 8)},
     {1, 512, 64, 3, {8, 8, 8}, 160, 2, 3, 1, K(double, 160, 3, 3, 512, 64, 2, 8, 8, 8)},

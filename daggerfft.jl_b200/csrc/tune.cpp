@@ -188,6 +188,13 @@ Pass tune_pass(const PassSpec& s) {
   return make_pass(t);
 }
 
+static double l2_bytes() {
+  int dev = 0, l2 = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+    l2 = 126 << 20;
+  return (double)l2;
+}
+
 int choose_slab(int dbl, int L, long long O, int inverse, const std::vector<Pass>& split,
                 unsigned flags) {
   std::ostringstream ko;
@@ -202,8 +209,15 @@ int choose_slab(int dbl, int L, long long O, int inverse, const std::vector<Pass
   std::vector<int> idx;
   const bool tune = (flags & DFFT_FLAG_TUNE) != 0;
   for (int v = 0; const SlabKernel* k = find_slab_kernel(dbl, L, v); ++v) {
-    // (an L2-resident array gains nothing from the single sweep of memory)
-    const bool dflt = k->dflt == 1 || (k->dflt == 2 && (double)L * L * (double)O * (dbl ? 16 : 8) >= 48e6);
+    // One sweep of memory instead of two, against the launch of the two
+    // per-axis passes, which overlap their neighbours.  384 (axes in three
+    // stages): from 48 MB, fft + ifft over (1, 2, 3), per-axis against fused:
+    // 28 MB 82 / 86 us, 48 MB 195 / 175, 113 MB 288 / 217.  192 (two stages):
+    // where input and output together exceed L2: 192^3 ComplexF32 (57 MB)
+    // 130 / 130 us back to back and less alone, dims (1, 2) of 70 MB 109 / 103,
+    // 192^3 ComplexF64 (113 MB) 259 / 236.
+    const double side = (double)L * L * (double)O * (dbl ? 16 : 8);
+    const bool dflt = k->dflt == 1 || (k->dflt == 2 && side >= 48e6) || (k->dflt == 3 && 2 * side > l2_bytes());
     if (!tune && !dflt && !(flags & DFFT_FLAG_FUSE)) continue;
     try {
       cands.push_back(make_slab_pass(dbl, L, O, inverse, v));

@@ -236,3 +236,21 @@ def test_inverse_scale_is_one_factor(L):
             r += float((np.abs(ref) ** 2).sum())
         e[flag] = (s / r) ** 0.5
     assert e[dfft.FLAG_FUSE] <= 1.02 * e[dfft.FLAG_NO_FUSE], e
+
+
+@pytest.mark.parametrize("L", [192, 384])
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+def test_default_rule_of_two_radix_lengths(L, dtype):
+    # 384 from 48 MB, 192 where input and output exceed L2: either side of the line
+    import torch
+    slab = L * L * np.dtype(dtype).itemsize
+    limit = 48e6 if L == 384 else torch.cuda.get_device_properties(0).L2_cache_size / 2
+    above = int(limit // slab) + 1
+    for O, fused in ((above - 1, False), (above, True)):
+        x = torch.empty((O, L, L), dtype=getattr(torch, np.dtype(dtype).name), device="cuda").permute(2, 1, 0)
+        for tag in (dfft.FFT(), dfft.IFFT()):
+            p = dfft.gpu_plan_transform(tag, x, (1, 2))
+            assert p.describe().startswith("slab-xy") == fused, (O, p.describe())
+    a = rand((L, L, above), dtype, seed=L)
+    F = dfft.fft(to_gpu(a), dims=(1, 2))
+    assert rel(to_np(F), np.fft.fft2(a.astype(np.complex128), axes=(0, 1))) <= tol_for(dtype)
