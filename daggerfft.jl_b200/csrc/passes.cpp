@@ -658,6 +658,8 @@ static Pass make_tiled_pass(const PassSpec& s) {
   if (occ < 1) throw Error{DFFT_ERROR_UNSUPPORTED_SIZE, "tiled kernel cannot be resident"};
   long long nb = (long long)sm_count() * occ;
   if (nb > g.ntiles) nb = g.ntiles;
+  // even rounds: as many CTAs as the rounds need
+  if (nb > 0) nb = (g.ntiles + (g.ntiles + nb - 1) / nb - 1) / ((g.ntiles + nb - 1) / nb);
   p.grid = dim3((unsigned)(nb > 0 ? nb : 1));
   return p;
 }

@@ -22,6 +22,12 @@
 // DCT-III, four passes, 54 us.)  The FFT runs in a padded complex work
 // buffer, one column per real column; columns stay independent of one
 // another.  Bounded waits as in the other pipelined passes.
+// Eight stage warps per SM: a tile's time is a chain of latencies, so the
+// loops over k are unrolled (their table and tile reads go out together) and
+// the planner launches no more CTAs than the rounds need.  256 x 256 Float64,
+// DCT-II + DCT-III of 20, 41 and 58 planes (1.1, 2.2 and 3.1 rounds of CTAs):
+// 49.0, 70.8 and 89.8 us with a round of k at a time on a full grid, 45.2,
+// 62.9 and 78.8 so; 46.4, 63.8 and 85.1 by FFTs of N points.
 #pragma once
 #include "real_pass.cuh"
 
@@ -64,7 +70,7 @@ __global__ void __launch_bounds__(LB, MINB)
   typedef typename cvec<T>::type V;
   constexpr int NC = C * P;
   constexpr int M = N / 2;                     // FFT length
-  constexpr int ROUNDS = M / 2 / P + 1;        // of the split / merge loops over k <= M/2
+  static_assert(M / 2 % P == 0, "whole rounds of the split / merge loops over k < M/2");
   constexpr int PS = N + 64 / (int)sizeof(T);  // contiguous tiles: elements between pencils (spread over the banks)
   static_assert(NC % 32 == 0 && NC + 32 == LB, "whole warps of stage threads plus one producer warp");
   static_assert(NB >= 2 && NB <= 4, "tile buffers");
@@ -182,10 +188,7 @@ __global__ void __launch_bounds__(LB, MINB)
       T* x = reinterpret_cast<T*>(buf) + (STRIDED ? c : c * PS);  // element n at x[n * S]
       const DctView<T, N, S> view{x};
       if constexpr (KIND == K_REDFT01) {
-#pragma unroll 1
-        for (int i = 0; i < ROUNDS; ++i) {
-          const int k = t + i * P;
-          if (k > M / 2) continue;
+        const auto merge = [&](int k) {
           const T xn = k == 0 ? (T)0 : x[(N - k) * S];
           const V A = cmul(ldg_c(cj + k), mk<V>(x[k * S], -xn));
           const V B = cconj(cmul(ldg_c(cj + M - k), mk<V>(x[(M - k) * S], -x[(M + k) * S])));
@@ -193,17 +196,17 @@ __global__ void __launch_bounds__(LB, MINB)
           const V Z = cadd(A, B);
           col.st(k, 0, cadd(Z, U));
           if (k > 0) col.st(M - k, 0, cconj(csub(Z, U)));
-        }
+        };
+#pragma unroll 4
+        for (int i = 0; i < M / 2 / P; ++i) merge(t + i * P);
+        if (t == 0) merge(M / 2);
         stage_sync<NC>();
         static_stages<T, M, P, 1, NC, DIR, 1, 1, 0, PadCol<V>, PadCol<V>, DctView<T, N, S>, GlobalTw<V>, Rs...>(
             d, t, col, col, view, tw, 0, 0, true);
       } else {
         static_stages<T, M, P, 1, NC, DIR, 1, 1, 0, DctView<T, N, S>, PadCol<V>, PadCol<V>, GlobalTw<V>, Rs...>(
             d, t, view, col, col, tw, 0, 0, true);
-#pragma unroll 1
-        for (int i = 0; i < ROUNDS; ++i) {
-          const int k = t + i * P;
-          if (k > M / 2) continue;
+        const auto split = [&](int k) {
           const V zk = col.ld(k, 0), zm = cconj(col.ld(k == 0 ? 0 : M - k, 0));
           const V E = cscale(cadd(zk, zm), (T)0.5);
           const V U = cmul(ldg_c(w + k), cscale(cmul_mi(csub(zk, zm)), (T)0.5));
@@ -213,7 +216,10 @@ __global__ void __launch_bounds__(LB, MINB)
           if (k > 0) x[(N - k) * S] = (T)-2 * q.y;
           x[(M - k) * S] = (T)2 * r.x;
           x[(M + k) * S] = k == 0 ? (T)2 * r.x : (T)-2 * r.y;
-        }
+        };
+#pragma unroll 4
+        for (int i = 0; i < M / 2 / P; ++i) split(t + i * P);
+        if (t == 0) split(M / 2);
       }
       fence_proxy_async_smem();  // the producer's store reads the tile next
       stage_sync<NC>();

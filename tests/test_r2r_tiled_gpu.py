@@ -70,3 +70,25 @@ def test_column_counts_that_do_not_fill_a_tile(n, cols, dtype, kind):
         y = to_np(dfft.fft(to_gpu(a), dims=(1,), transforms=tr))
         assert np.isfinite(y[:, :-1]).all() and not np.isfinite(y[:, -1]).all()
         assert rel(y[:, :-1], np.asarray(ref)[:, :-1]) <= tol_for(dtype)
+
+
+@pytest.mark.parametrize("n", [128, 256, 512])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", [dfft.REDFT10, dfft.REDFT01])
+@pytest.mark.parametrize("shape_of", [lambda n: ((n, 9479), (1,)), lambda n: ((20, n, 300), (2,))])
+def test_several_rounds_of_tiles(n, dtype, kind, shape_of):
+    # more tiles than CTAs, in rounds that are not full
+    shape, dims = shape_of(n)
+    a = rand(shape, dtype, seed=n)
+    p = dfft.gpu_plan_transform(dfft.R2R((kind,)), to_gpu(a), dims)
+    assert p.describe().startswith("tiled"), p.describe()
+    y = to_np(dfft.fft(to_gpu(a), dims=dims, transforms=(dfft.R2R((kind,)),)))
+    k, m = np.arange(n)[:, None], np.arange(n)[None, :]
+    if kind == dfft.REDFT10:
+        t = 2 * np.cos(np.pi / n * k * (m + 0.5))
+    else:
+        t = 2 * np.cos(np.pi / n * (k + 0.5) * m)
+        t[:, 0] = 1
+    ref = np.moveaxis(np.tensordot(t, a.astype(np.float64), axes=(1, dims[0] - 1)), 0, dims[0] - 1)
+    assert rel(y, ref) <= tol_for(dtype)
+    assert dfft.device_error() == 0
