@@ -25,31 +25,27 @@
 
 namespace dfft {
 
-// Columns of the tile a thread helps to move, and its elements of them, so
+// The column of the tile a thread helps to move, and its elements of it, so
 // that consecutive lanes touch consecutive memory of that side.  Columns
-// side by side (cfast): one column per thread, elements nthreads / C apart.
-// Unit stride along the column (the contiguous axis, and the output of a
-// four-step axis's first pass): the column's share of the threads walks it, or
-// groups of G lanes do where that is less than a warp (fft + ifft of one
-// column of 5003 ComplexF32 points: 405 us with 32 lanes at work, 153 with all;
-// 40 Float32 pencils of 1002 points, rfft + irfft: 48 us, 118 with the side maps inside the stages).
+// side by side (cfast): elements nthreads / C apart.  Unit stride along the
+// column (the contiguous axis, and the output of a four-step axis's first
+// pass): the column's share of the threads, in order (fft + ifft of one column
+// of 5003 ComplexF32 points: 405 us with one group of 32 lanes per column at
+// work, 153 so; irfft of 29547 x 25 Float64 44 us, its columns taking turns,
+// and 15).
 struct TileLanes {
-  int c, cstep, k, kstep;
+  int c, k, kstep;
 };
-__device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, const IoAny& io, int L) {
-  const int tid = threadIdx.x, n = blockDim.x;
-  if (d.cfast && io.sk != 1) return TileLanes{tid % d.C, d.C, tid / d.C, n / d.C};
-  const int share = n / d.C;
-  if (share >= 32) return TileLanes{tid / share, n / share, tid % share, share};
-  int G = 1;
-  while (G < 32 && G < L && G * 2 <= n) G *= 2;
-  const int groups = n / G;  // a remainder of n mod G threads moves nothing
-  const int g = tid / G;
-  return TileLanes{g < groups ? g : d.C, groups, tid % G, G};
+__device__ __forceinline__ TileLanes tile_lanes(const PassDesc& d, const IoAny& io) {
+  const int tid = threadIdx.x, share = blockDim.x / d.C;
+  if (d.cfast && io.sk != 1) return TileLanes{tid % d.C, tid / d.C, share};
+  return TileLanes{tid / share, tid % share, share};
 }
 
-constexpr int kAnyBatch = 8;  // elements in flight per thread
-constexpr int kR2RBatch = 2;  // the r2r kinds: their maps are longer, and there are nine of them
+// Elements in flight per thread.  (Eight execute twice the code for nothing
+// where a thread has three or four: rfft of 200000 x 81 Float32 258 us, 223
+// with four.)
+constexpr int kAnyBatch = 4;
 
 // Elements k, k + ks, ... < L of one column: get(k) from memory, times the
 // chirp or filter where the side has one (zero beyond the chirp), conjugated
@@ -163,7 +159,7 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
   typedef typename cvec<T>::type V;
   __builtin_assume(__isShared(sm));
   const IoAny& io = d.in;
-  const TileLanes ln = tile_lanes(d, io, L);
+  const TileLanes ln = tile_lanes(d, io);
   const bool inv = d.inverse != 0;
   const V* pc = reinterpret_cast<const V*>(io.p);
   const T* pr = reinterpret_cast<const T*>(io.p);
@@ -171,58 +167,56 @@ __device__ __noinline__ void tile_load(const PassDesc& d, typename cvec<T>::type
   const long long sk = io.sk;
   const int io_n = io.n;
   const T z = (T)0;
-  for (int c = ln.c; c < d.C; c += ln.cstep) {
-    const long long q = (long long)blockIdx.x * d.C + c;
-    if (q >= d.Q) break;
-    const long long b = column_base(io, d.I, q);
-    // index along the whole axis of the column's element 0 (four-step sub-axes)
-    const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
-    V* col = sm + (size_t)c * d.ld;
-    auto in = [&](auto get) { column_in<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, get); };
-    switch (io.kind) {
-      case IO_CPLX:
-        in([=](int k) { return pc[b + k * sk]; });
-        break;
-      case IO_REAL_PAIR:
-        if (sk == 1 && whole_pairs(pr + b)) in([=](int k) { return *reinterpret_cast<const V*>(pr + b + 2 * (long long)k); });
-        else in([=](int k) { return mk<V>(pr[b + (2 * k) * sk], pr[b + (2 * k + 1) * sk]); });
-        break;
-      case IO_REAL:
-        in([=](int k) { return mk<V>(pr[b + k * sk], z); });
-        break;
-      case IO_HERM_PAIR:
-        // even-length C2R pre-pass: Z'_k = (A + B) + i conj(w^k) (A - B),
-        // A = X_k, B = conj(X_{n-k}) (Im X_0 and Im X_n ignored); the inverse
-        // FFT of Z' (length n) interleaves to 2n * x
-        if (w) in([=](int k) { return herm_pair(pc[b + k * sk], pc[b + (io_n - k) * sk], cconj(ldg_c(w + k)), k); });
-        else in([=](int k) {  // exp(+2 pi i k / (2n)), computed in the kernel
-          double sn, cs;
-          sincospi((double)k / (double)io_n, &sn, &cs);
-          return herm_pair(pc[b + k * sk], pc[b + (io_n - k) * sk], mk<V>((T)cs, (T)sn), k);
-        });
-        break;
-      case IO_HERM_FULL: {
-        const WholeAxis a = whole_axis(io, b);
-        in([=](int k) {
-          const int kf = a.at(k);
-          if (kf == 0) return mk<V>(pc[a.b].x, z);  // c2r ignores Im X_0
-          if (2 * kf <= io_n) return pc[a.b + kf * a.s];
-          return cconj(pc[a.b + (io_n - kf) * a.s]);
-        });
-        break;
-      }
-      default: {
-        const WholeAxis a = whole_axis(io, b);
-        auto in = [&](auto get) { column_in<T, kR2RBatch>(io, inv, j, col, ln.k, ln.kstep, L, get); };
+  const int c = ln.c;
+  const long long q = (long long)blockIdx.x * d.C + c;
+  if (q >= d.Q) return;
+  const long long b = column_base(io, d.I, q);
+  // index along the whole axis of the column's element 0 (four-step sub-axes)
+  const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
+  V* col = sm + (size_t)c * d.ld;
+  auto in = [&](auto get) { column_in<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, get); };
+  switch (io.kind) {
+    case IO_CPLX:
+      in([=](int k) { return pc[b + k * sk]; });
+      break;
+    case IO_REAL_PAIR:
+      if (sk == 1 && whole_pairs(pr + b)) in([=](int k) { return *reinterpret_cast<const V*>(pr + b + 2 * (long long)k); });
+      else in([=](int k) { return mk<V>(pr[b + (2 * k) * sk], pr[b + (2 * k + 1) * sk]); });
+      break;
+    case IO_REAL:
+      in([=](int k) { return mk<V>(pr[b + k * sk], z); });
+      break;
+    case IO_HERM_PAIR:
+      // even-length C2R pre-pass: Z'_k = (A + B) + i conj(w^k) (A - B),
+      // A = X_k, B = conj(X_{n-k}) (Im X_0 and Im X_n ignored); the inverse
+      // FFT of Z' (length n) interleaves to 2n * x
+      if (w) in([=](int k) { return herm_pair(pc[b + k * sk], pc[b + (io_n - k) * sk], cconj(ldg_c(w + k)), k); });
+      else in([=](int k) {  // exp(+2 pi i k / (2n)), computed in the kernel
+        double sn, cs;
+        sincospi((double)k / (double)io_n, &sn, &cs);
+        return herm_pair(pc[b + k * sk], pc[b + (io_n - k) * sk], mk<V>((T)cs, (T)sn), k);
+      });
+      break;
+    case IO_HERM_FULL: {
+      const WholeAxis a = whole_axis(io, b);
+      in([=](int k) {
+        const int kf = a.at(k), m = 2 * kf <= io_n ? kf : io_n - kf;
+        V v = pc[a.b + m * a.s];
+        if (kf == 0) v.y = z;  // c2r ignores Im X_0
+        return m == kf ? v : cconj(v);
+      });
+      break;
+    }
+    default: {
+      const WholeAxis a = whole_axis(io, b);
 #define DFFT_R2R_IN(KIND) \
   case KIND: in([=](int k) { return r2r_load<T, KIND>(pr, a.b, a.s, io_n, w, a.at(k)); }); break;
-        switch (io.r2r) {
-          DFFT_R2R_IN(K_REDFT10) DFFT_R2R_IN(K_RODFT10) DFFT_R2R_IN(K_REDFT01) DFFT_R2R_IN(K_RODFT01)
-          DFFT_R2R_IN(K_REDFT11) DFFT_R2R_IN(K_RODFT11) DFFT_R2R_IN(K_REDFT00) DFFT_R2R_IN(K_RODFT00)
-          default: in([=](int k) { return r2r_load<T, K_DHT>(pr, a.b, a.s, io_n, w, a.at(k)); }); break;
-        }
-#undef DFFT_R2R_IN
+      switch (io.r2r) {
+        DFFT_R2R_IN(K_REDFT10) DFFT_R2R_IN(K_RODFT10) DFFT_R2R_IN(K_REDFT01) DFFT_R2R_IN(K_RODFT01)
+        DFFT_R2R_IN(K_REDFT11) DFFT_R2R_IN(K_RODFT11) DFFT_R2R_IN(K_REDFT00) DFFT_R2R_IN(K_RODFT00)
+        default: in([=](int k) { return r2r_load<T, K_DHT>(pr, a.b, a.s, io_n, w, a.at(k)); }); break;
       }
+#undef DFFT_R2R_IN
     }
   }
 }
@@ -232,81 +226,77 @@ __device__ __noinline__ void tile_store(const PassDesc& d, const typename cvec<T
   typedef typename cvec<T>::type V;
   __builtin_assume(__isShared(sm));
   const IoAny& io = d.out;
-  const TileLanes ln = tile_lanes(d, io, L);
+  const TileLanes ln = tile_lanes(d, io);
   const bool inv = d.inverse != 0 || d.epi == kEpiChirp;
   V* pc = reinterpret_cast<V*>(io.p);
   T* pr = reinterpret_cast<T*>(io.p);
   const V* w = reinterpret_cast<const V*>(io.w);
   const long long sk = io.sk;
   const T s = (T)d.scale;
-  for (int c = ln.c; c < d.C; c += ln.cstep) {
-    const long long q = (long long)blockIdx.x * d.C + c;
-    if (q >= d.Q) break;
-    const long long b = column_base(io, d.I, q);
-    const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
-    const V* col = sm + (size_t)c * d.ld;
-    auto out = [&](int n, auto put) { column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, n, NoFactor{}, put); };
-    if (d.epi == 1) {
-      // R2C post-pass over the half-length spectrum Z (length M = L):
-      // X_k = E_k + w^k O_k, E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2
-      const V* w2 = reinterpret_cast<const V*>(d.tw2);
-      for (int k = ln.k; k <= L; k += ln.kstep) {
-        const V zk = col[swz<V>(k == L ? 0 : k)];
-        const V zm = cconj(col[swz<V>(k == 0 ? 0 : L - k)]);
-        const V e = cscale(cadd(zk, zm), (T)0.5);
-        const V o = cscale(cmul_mi(csub(zk, zm)), (T)0.5);
-        pc[b + k * sk] = cscale(cadd(e, cmul(ldg_c(w2 + k), o)), s);
-      }
-      continue;
+  const int c = ln.c;
+  const long long q = (long long)blockIdx.x * d.C + c;
+  if (q >= d.Q) return;
+  const long long b = column_base(io, d.I, q);
+  const long long j = io.t_m > 0 ? (b % io.t_ia) / io.t_i : 0;
+  const V* col = sm + (size_t)c * d.ld;
+  auto out = [&](int n, auto put) { column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, n, NoFactor{}, put); };
+  if (d.epi == 1) {
+    // R2C post-pass over the half-length spectrum Z (length M = L):
+    // X_k = E_k + w^k O_k, E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2
+    const V* w2 = reinterpret_cast<const V*>(d.tw2);
+    for (int k = ln.k; k <= L; k += ln.kstep) {
+      const V zk = col[swz<V>(k == L ? 0 : k)];
+      const V zm = cconj(col[swz<V>(k == 0 ? 0 : L - k)]);
+      const V e = cscale(cadd(zk, zm), (T)0.5);
+      const V o = cscale(cmul_mi(csub(zk, zm)), (T)0.5);
+      pc[b + k * sk] = cscale(cadd(e, cmul(ldg_c(w2 + k), o)), s);
     }
-    switch (io.kind) {
-      case IO_CPLX:
-        out(L, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
-        break;
-      case IO_TRUNC: {
-        const long long tm = io.t_m > 0 ? io.t_m : 1;
-        const int last = io.n;
-        out(L, [=](int k, V v) {
-          if (j + tm * k <= last) pc[b + k * sk] = cscale(v, s);
-        });
-        break;
-      }
-      case IO_CPLX_TW: {
-        const unsigned jj = (unsigned)((b % io.t_ia) / io.t_i);
-        const int sh = io.n;
-        const V* hi = w + (1 << sh);
-        const auto twiddle = [=](int k) {
-          const unsigned m = jj * (unsigned)k;
-          return split_twiddle(ldg_c(w + (m & ((1u << sh) - 1))), hi + 2 * (m >> sh));
-        };
-        column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, twiddle, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
-        break;
-      }
-      case IO_REAL_PAIR:
-        if (sk == 1 && whole_pairs(pr + b)) out(L, [=](int k, V v) { *reinterpret_cast<V*>(pr + b + 2 * (long long)k) = cscale(v, s); });
-        else out(L, [=](int k, V v) {
-          pr[b + (2 * k) * sk] = v.x * s;
-          pr[b + (2 * k + 1) * sk] = v.y * s;
-        });
-        break;
-      case IO_REAL:
-        out(L, [=](int k, V v) { pr[b + k * sk] = v.x * s; });
-        break;
-      default: {
-        const WholeAxis a = whole_axis(io, b);
-        const int N = io.n;
-        auto out = [&](int n, auto put) {
-          column_out<T, kR2RBatch>(io, inv, j, col, ln.k, ln.kstep, n, NoFactor{}, put);
-        };
+    return;
+  }
+  switch (io.kind) {
+    case IO_CPLX:
+      out(L, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
+      break;
+    case IO_TRUNC: {
+      const long long tm = io.t_m > 0 ? io.t_m : 1;
+      const int last = io.n;
+      out(io.t_m > 0 ? L : last + 1, [=](int k, V v) {
+        if (j + tm * k <= last) pc[b + k * sk] = cscale(v, s);
+      });
+      break;
+    }
+    case IO_CPLX_TW: {
+      const unsigned jj = (unsigned)((b % io.t_ia) / io.t_i);
+      const int sh = io.n;
+      const V* hi = w + (1 << sh);
+      const auto twiddle = [=](int k) {
+        const unsigned m = jj * (unsigned)k;
+        return split_twiddle(ldg_c(w + (m & ((1u << sh) - 1))), hi + 2 * (m >> sh));
+      };
+      column_out<T, kAnyBatch>(io, inv, j, col, ln.k, ln.kstep, L, twiddle, [=](int k, V v) { pc[b + k * sk] = cscale(v, s); });
+      break;
+    }
+    case IO_REAL_PAIR:
+      if (sk == 1 && whole_pairs(pr + b)) out(L, [=](int k, V v) { *reinterpret_cast<V*>(pr + b + 2 * (long long)k) = cscale(v, s); });
+      else out(L, [=](int k, V v) {
+        pr[b + (2 * k) * sk] = v.x * s;
+        pr[b + (2 * k + 1) * sk] = v.y * s;
+      });
+      break;
+    case IO_REAL:
+      out(L, [=](int k, V v) { pr[b + k * sk] = v.x * s; });
+      break;
+    default: {
+      const WholeAxis a = whole_axis(io, b);
+      const int N = io.n;
 #define DFFT_R2R_OUT(KIND) \
   case KIND: out(L, [=](int k, V v) { r2r_store<T, KIND>(pr, a.b, a.s, N, w, a.at(k), v, s); }); break;
-        switch (io.r2r) {
-          DFFT_R2R_OUT(K_REDFT10) DFFT_R2R_OUT(K_RODFT10) DFFT_R2R_OUT(K_REDFT01) DFFT_R2R_OUT(K_RODFT01)
-          DFFT_R2R_OUT(K_REDFT11) DFFT_R2R_OUT(K_RODFT11) DFFT_R2R_OUT(K_REDFT00) DFFT_R2R_OUT(K_RODFT00)
-          default: out(L, [=](int k, V v) { r2r_store<T, K_DHT>(pr, a.b, a.s, N, w, a.at(k), v, s); }); break;
-        }
-#undef DFFT_R2R_OUT
+      switch (io.r2r) {
+        DFFT_R2R_OUT(K_REDFT10) DFFT_R2R_OUT(K_RODFT10) DFFT_R2R_OUT(K_REDFT01) DFFT_R2R_OUT(K_RODFT01)
+        DFFT_R2R_OUT(K_REDFT11) DFFT_R2R_OUT(K_RODFT11) DFFT_R2R_OUT(K_REDFT00) DFFT_R2R_OUT(K_RODFT00)
+        default: out(L, [=](int k, V v) { r2r_store<T, K_DHT>(pr, a.b, a.s, N, w, a.at(k), v, s); }); break;
       }
+#undef DFFT_R2R_OUT
     }
   }
 }

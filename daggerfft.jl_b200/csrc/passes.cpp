@@ -917,6 +917,7 @@ Pass make_pass(const PassSpec& s) {
     } else {
       C = 1;
       while (C * 2 * P <= 256) C *= 2;
+      while (C > 1 && C * P > 64 && (Q + C - 1) / C < sm_count()) C /= 2;
     }
   }
   while (C > 1 && (C * P > lb || (size_t)C * col_bytes > smax)) C /= 2;

@@ -100,3 +100,17 @@ def _smooth5(k):
         while k % q == 0:
             k //= q
     return k == 1
+
+
+@pytest.mark.parametrize("n", [17, 23, 37, 73, 137, 151, 311, 613, 1123, 1217, 1531, 1777])
+@pytest.mark.parametrize("strided", [False, True])
+def test_every_compiled_convolution_on_real_sides(n, strided):
+    # one length behind each convolution of the general kernel that the
+    # complex two-radix kernels do not use
+    shape, dims = ((5, n, 3), (2,)) if strided else ((n, 7), (1,))
+    for dtype in (np.float32, np.float64):
+        a = rand(shape, dtype, seed=n)
+        g = to_gpu(a)
+        F = dfft.rfft(g, dims=dims)
+        assert rel(to_np(F), oracle.rfft(a, dims=dims)) <= tol_for(dtype)
+        assert rel(to_np(dfft.irfft(F, n, dims=dims)), a) <= tol_for(dtype)
