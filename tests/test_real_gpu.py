@@ -75,3 +75,19 @@ def test_few_contiguous_pencils(n, cols, dtype):
     y = dfft.fft(to_gpu(a), dims=(1,), transforms=(dfft.R2R((dfft.DHT,)),))
     h = np.fft.fft(a.astype(np.complex128), axis=0)
     assert rel(to_np(y), h.real - h.imag) <= tol_for(dtype)
+
+
+@pytest.mark.parametrize("n", [9, 27, 45, 81, 105, 243])
+@pytest.mark.parametrize("cols", [1, 129, 300])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_odd_contiguous_pencils(n, cols, dtype):
+    # columns of unit stride with real, truncated and Hermitian sides and no
+    # chirp: shares of the threads below the batch of elements in flight, last
+    # batches that are part of a column, a last tile that is part of a tile;
+    # a strided copy of the same columns takes the general form of the sides
+    a = rand((n, cols), dtype, seed=n + cols)
+    F = dfft.rfft(to_gpu(a), dims=(1,))
+    assert rel(to_np(F), oracle.rfft(a, dims=(1,))) <= tol_for(dtype)
+    assert rel(to_np(dfft.irfft(F, n, dims=(1,))), a) <= tol_for(dtype)
+    Fs = dfft.rfft(to_gpu(np.ascontiguousarray(a.T)), dims=(2,))
+    assert rel(to_np(Fs).T, to_np(F)) <= tol_for(dtype)
