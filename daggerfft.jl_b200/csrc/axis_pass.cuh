@@ -122,7 +122,8 @@ template <typename V> __device__ __forceinline__ V ldg_c(const V* p) { return __
 // rounds at full size, as in a table of all N entries: at most 0.63 units of
 // the last place, against 1.4 for the product of two rounded entries (relative
 // error of a 2^18-point Float32 rfft 1.50e-7 and 1.53e-7, of 2^20 ComplexF32
-// points 1.67e-7 and 1.69e-7, at the same time, 29.5 us fft + ifft).
+// points 1.67e-7 and 1.69e-7; one fft of 2^20 points 14.1 us either way, of
+// 2^18 11.4 against 10.4, of 45000 6.4 against 6.0).
 template <typename V> __device__ __forceinline__ V split_twiddle(V lo, const V* hi) {
   V h, r;
   if constexpr (sizeof(V) == 8) {
@@ -136,8 +137,8 @@ template <typename V> __device__ __forceinline__ V split_twiddle(V lo, const V* 
   return cadd(h, cadd(r, cmul(h, lo)));
 }
 
-// Every pass kernel calls this before its first access to the arrays, from
-// all threads: it waits until the kernels before it in the stream are
+// Every pass kernel but mixed_pass (launched in the ordinary way) calls this
+// before its first access to the arrays, from all threads: it waits until the kernels before it in the stream are
 // complete and visible, then lets the next one be scheduled.  The passes of
 // a transform are launched with programmatic stream serialization, so the
 // next pass's launch and set-up overlap this one's tail instead of following
